@@ -80,6 +80,14 @@ static int ctx_alloc(Ctx *c) {
         for (int k = 3; k < 9; k++) o_mg[l][k] = carve(m * sizeof(float)); // aE, aN, dP, wD, x0, x1
         o_mg[l][9] = carve(m * sizeof(float) + m);                       // b, then act bytes
     }
+    size_t vec_bytes = 0;
+    for (const ResPlan &P : c->res) {
+        if (!P.blocks) continue;
+        c->res_red_bytes = std::max(c->res_red_bytes, res_red_bytes(P));
+        c->res_halo_bytes = std::max(c->res_halo_bytes, res_halo_bytes(P));
+        vec_bytes = std::max(vec_bytes, res_vec_bytes(P));
+    }
+    const size_t o_red = carve(c->res_red_bytes), o_halo = carve(c->res_halo_bytes), o_vec = carve(vec_bytes);
     size_t o_part = carve((size_t)kMaxRedValues * c->max_blocks * sizeof(double));
     size_t o_cnt = carve(64);
     size_t o_dev = carve(sizeof(DevScalars));
@@ -117,6 +125,9 @@ static int ctx_alloc(Ctx *c) {
         m.b = (float *)(b + o_mg[l][9]);
         m.act = (uint8_t *)(b + o_mg[l][9] + cnt * sizeof(float));
     }
+    c->res_red = (uint4 *)(b + o_red);
+    c->res_halo = (uint4 *)(b + o_halo);
+    c->res_vec = (double2 *)(b + o_vec);
     c->partials = (double *)(b + o_part);
     c->counter = (unsigned int *)(b + o_cnt);
     c->dev = (DevScalars *)(b + o_dev);
@@ -271,6 +282,12 @@ SHK_API int shk_create(int nx, int ny, double lx, double ly, void *stream, void 
         c->graph_mode = std::min(2, std::max(0, atoi(v)));
         c->graphs_disabled = c->graph_mode == 0;
     }
+    // SHK_CG_RESIDENT=0: the Jacobi and Chebyshev solves of small grids by the general kernels too (as
+    // SHK_MG_TMA=0, which asks for the row-marching CG kernels, implies)
+    const char *resident = getenv("SHK_CG_RESIDENT");
+    if (resident ? atoi(resident) != 0 : c->mg_tma)
+        for (int k = 0; k < 2; k++) c->res[k] = res_plan(nx, ny, c->num_sms, k == 1);
+    if (const char *v = getenv("SHK_TEST_RESIDENT_POLLS")) c->res_spin = std::max(0L, atol(v));
     c->max_blocks = c->grid_stencil > c->march_blocks ? c->grid_stencil : c->march_blocks;
     if (c->max_blocks < c->num_sms * 8) c->max_blocks = c->num_sms * 8;
     rc = mg_set_first_wait_polls();
@@ -542,16 +559,18 @@ SHK_API int shk_picard_solve(void *ctx, const shk_picard_opts *po, const shk_cg_
         c->assembled_parabolic = false;
         shk_cg_stats cs;
         memset(&cs, 0, sizeof(cs));
-        rc = run_cg(c, o, &cs);
+        bool deferred = false;
+        rc = run_cg(c, o, &cs, &deferred);
         if (rc) return rc;
-        s.cg_iters_total += cs.niter;
-        s.cg_solves++;
-        if (cs.status == SHK_BREAKDOWN) s.cg_breakdowns++;
         if (relax && (rc = launch_relax(c, po->alpha, c->h_prev))) return rc;
         const bool check = (iter % check_every == 0) || iter == po->iters;
         if ((rc = launch_tail(c, check))) return rc;
+        if ((deferred || check) && (rc = read_scalars(c))) return rc;
+        if (deferred && (rc = collect_cg(c, o, &cs))) return rc;
+        s.cg_iters_total += cs.niter;
+        s.cg_solves++;
+        if (cs.status == SHK_BREAKDOWN) s.cg_breakdowns++;
         if (check) {
-            if ((rc = read_scalars(c))) return rc;
             s.max_dh = c->host_dev->pic.dmax;
             s.max_h = c->host_dev->pic.hmax;
             if (s.max_dh / (s.max_h + DBL_EPSILON) < po->tol) {

@@ -85,6 +85,14 @@ struct DevScalars {
     ChebDev cheb;
     PicDev pic;
     double ref_rr, ref_bb; // mixed precision: outer residual norms
+    unsigned int res_epoch; // resident solve: exchange tags used so far
+    unsigned int pad;
+};
+
+// Geometry of the resident solve (shk_resident.cu): rows per thread, threads per row group, row
+// groups per block, blocks (0: the grid does not fit).
+struct ResPlan {
+    int rows = 0, txp = 0, ty = 0, blocks = 0;
 };
 
 // One level of the multigrid hierarchy (level 0 aliases the Float32 operator of the mixed form).
@@ -159,6 +167,12 @@ struct Ctx {
     bool mg_pair_x = true;    // the outer CG's x updated once per two iterations (bit-identical x)
     struct MgTma *mg_maps = nullptr;  // the levels' tensor maps (built on first use)
     struct CgTma *cg_maps = nullptr;  // the plain Jacobi CG's tensor maps (built before its first capture)
+    ResPlan res[2];           // the resident solve's geometry, Jacobi and Chebyshev (blocks = 0: does not fit)
+    size_t res_red_bytes = 0, res_halo_bytes = 0;
+    uint4 *res_red = nullptr, *res_halo = nullptr;  // its exchange buffers
+    double2 *res_vec = nullptr;                     // its scratch vectors
+    bool res_restart = false; // its tags start over at the next solve
+    long res_spin = 1L << 21; // polls before one of its waits gives up
     int max_blocks = 0;
     int grid_stencil = 0;    // blocks for tile-stride kernels
     int march_th = 8;        // row-marching tile height
@@ -247,11 +261,20 @@ int launch_matvec(Ctx *c, const double *x, double *y);
 int run_chebyshev_bounds(Ctx *c, int nsteps, const double *rhs);
 int cheb_set_bounds(Ctx *c, double lmin, double lmax);
 int launch_chebyshev_apply_standalone(Ctx *c, int degree, const double *x, double *y);
-int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st);
+int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred = nullptr);
+int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st);
 int read_scalars(Ctx *c);
 int move_scalars(Ctx *c, void *dst, const void *src, size_t bytes, bool to_host);
 int residual_norms(Ctx *c, const double *x, double *rnorm, double *bnorm);
 int jacobi_smooth(Ctx *c, double *x, double *tmp, int sweeps, double omega);
+
+// shk_resident.cu
+ResPlan res_plan(int nx, int ny, int num_sms, bool cheb);
+size_t res_red_bytes(const ResPlan &P);
+size_t res_halo_bytes(const ResPlan &P);
+size_t res_vec_bytes(const ResPlan &P);
+bool res_serves(const Ctx *c, const shk_cg_opts *o);
+int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0);
 
 // ensemble kernels: shk_fields.cu
 void ens_assemble(cudaStream_t s, EnsInst *E, const int *b2i, int nblocks);

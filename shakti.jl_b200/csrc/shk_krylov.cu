@@ -24,6 +24,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include "shk_cheb.cuh"
 #include "shk_device.cuh"
 
 namespace shk {
@@ -498,94 +499,29 @@ __global__ void __launch_bounds__(kThreads) k_cheb(int nx, int ny, const T *__re
     }
 }
 
-// Chebyshev per-step coefficients from the bounds (src/preconditioner.jl:241-263).
-__device__ void cheb_tables(ChebDev *ch) {
-    const double d_mid = (ch->lam_max + ch->lam_min) / 2;
-    const double c_rad = (ch->lam_max - ch->lam_min) / 2;
-    double alpha = 1.0 / d_mid;
-    ch->calpha[1] = alpha;
-    ch->cbeta[1] = 0.0;
-    double alpha_prev = alpha;
-    for (int k = 2; k <= kMaxChebDegree; k++) {
-        double t = c_rad * alpha_prev / 2;
-        double beta = t * t;
-        alpha = 1.0 / (d_mid - beta / alpha_prev);
-        ch->calpha[k] = alpha;
-        ch->cbeta[k] = beta;
-        alpha_prev = alpha;
-    }
-}
-
 __global__ void k_cheb_set_bounds(ChebDev *ch, double lmin, double lmax) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         ch->lam_min = lmin;
         ch->lam_max = lmax;
-        cheb_tables(ch);
+        cheb_coefficients(lmin, lmax, kMaxChebDegree, ch->calpha, ch->cbeta);
     }
 }
 
-// Sturm count of eigenvalues below x for SymTridiagonal(d, e).
-__device__ int sturm(int m, const double *d, const double *e, double x) {
-    int cnt = 0;
-    double q = d[0] - x;
-    if (q < 0) cnt++;
-    for (int i = 1; i < m; i++) {
-        if (q == 0) q = DBL_EPSILON * (fabs(e[i - 1]) + DBL_MIN);
-        q = d[i] - x - e[i - 1] * e[i - 1] / q;
-        if (q < 0) cnt++;
-    }
-    return cnt;
-}
-
-// estimate_eigenvalue_bounds tail + update_chebyshev_bounds! validity/fallback
-// (src/preconditioner.jl:115-133, 219-230).  LAPACK's eigvals(SymTridiagonal) is replaced by
-// bisection on the Sturm count for the two extreme eigenvalues (the only ones used).
+// The estimate after m Lanczos steps and update_chebyshev_bounds!'s validity test and fallback, by
+// one warp.
 __device__ void cheb_finish_estimate(ChebDev *ch, int m) {
-    double d[kMaxChebSteps], e[kMaxChebSteps];
-    d[0] = 1 / ch->alphas[0];
-    for (int k = 1; k < m; k++) d[k] = 1 / ch->alphas[k] + ch->betas[k - 1] / ch->alphas[k - 1];
-    for (int k = 0; k < m - 1; k++) e[k] = sqrt(ch->betas[k]) / ch->alphas[k];
-    bool finite = true;
-    for (int k = 0; k < m; k++) finite = finite && isfinite(d[k]);
-    for (int k = 0; k < m - 1; k++) finite = finite && isfinite(e[k]);
-    double lmin = __longlong_as_double(0x7ff8000000000000LL), lmax = lmin;
-    if (finite) {
-        double lo = INFINITY, hi = -INFINITY;
-        for (int i = 0; i < m; i++) {
-            double rad = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < m ? fabs(e[i]) : 0.0);
-            lo = fmin(lo, d[i] - rad);
-            hi = fmax(hi, d[i] + rad);
-        }
-        double span = fmax(fabs(lo), fabs(hi));
-        lo -= DBL_EPSILON * span + DBL_MIN;
-        hi += DBL_EPSILON * span + DBL_MIN;
-        double a = lo, b = hi;
-        for (int it = 0; it < 200; it++) {
-            double mid = 0.5 * (a + b);
-            if (mid == a || mid == b) break;
-            if (sturm(m, d, e, mid) >= 1) b = mid; else a = mid;
-        }
-        double rmin = 0.5 * (a + b);
-        a = lo;
-        b = hi;
-        for (int it = 0; it < 200; it++) {
-            double mid = 0.5 * (a + b);
-            if (mid == a || mid == b) break;
-            if (sturm(m, d, e, mid) >= m) b = mid; else a = mid;
-        }
-        double rmax = 0.5 * (a + b);
-        lmin = rmin * 0.9;
-        lmax = rmax * 1.1;
-    }
+    __shared__ double d[kMaxChebSteps], e[kMaxChebSteps];
+    double lmin, lmax;
+    cheb_bounds_warp(ch->alphas, ch->betas, m, d, e, lmin, lmax);
+    if (threadIdx.x != 0) return;
     ch->est_min = lmin;
     ch->est_max = lmax;
-    const bool ok = isfinite(lmin) && isfinite(lmax) && lmin > 0 && lmax > lmin;
-    ch->adopted = ok;
-    if (ok) {
+    ch->adopted = cheb_bounds_ok(lmin, lmax);
+    if (ch->adopted) {
         ch->lam_min = lmin;
         ch->lam_max = lmax;
     }
-    cheb_tables(ch);
+    cheb_coefficients(ch->lam_min, ch->lam_max, kMaxChebDegree, ch->calpha, ch->cbeta);
 }
 
 // Lanczos-from-CG estimate (src/preconditioner.jl:89-113), step k of nsteps:
@@ -613,9 +549,12 @@ __global__ void __launch_bounds__(kThreads) k_est_A(int nx, int ny, const double
         if (FIRST) red[1] += pc * pc;
     }
     double out[2];
-    if (grid_reduce<2, false>(red, partials, counter, out) && threadIdx.x == 0) {
-        if (FIRST) ch->gamma = out[1];
-        ch->alphas[k] = ch->gamma / out[0];
+    if (grid_reduce<2, false>(red, partials, counter, out) && threadIdx.x < 32) {
+        if (threadIdx.x == 0) {
+            if (FIRST) ch->gamma = out[1];
+            ch->alphas[k] = ch->gamma / out[0];
+        }
+        __syncwarp();
         if (k == nsteps - 1) cheb_finish_estimate(ch, nsteps);
     }
 }
@@ -1110,7 +1049,32 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
     return SHK_OK;
 }
 
-int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
+// A Float64 solve's outcome from the scalars last read back.
+int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
+    const CgDev &g = c->host_dev->cg;
+    if (g.fault) {
+        c->res_restart = true;
+        return fail(c, SHK_CUDA_ERROR, res_serves(c, o)
+                                           ? "an exchange of the resident solve did not complete (bounded wait ran out)"
+                                           : "a TMA tile copy did not complete (bounded wait ran out)");
+    }
+    memset(st, 0, sizeof(*st));
+    st->niter = (long)g.iter;
+    st->status = g.status;
+    st->rnorm0 = g.rnorm0;
+    st->rnorm = g.rnorm;
+    if (o->precond == SHK_PRECOND_CHEBYSHEV) {
+        st->lambda_min = c->host_dev->cheb.lam_min;
+        st->lambda_max = c->host_dev->cheb.lam_max;
+        st->bounds_valid = c->host_dev->cheb.adopted;
+    }
+    return SHK_OK;
+}
+
+// With `deferred`, a solve may return before it has finished (*deferred set): the caller reads the
+// scalars after the work it queues next and calls collect_cg.
+int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
+    if (deferred) *deferred = false;
     const int nx = c->nx, ny = c->ny, n = nx * ny;
     const double *ws = c->ws_x0;  // consumed by this solve (Float64 forms; ignored by the mixed form)
     c->ws_x0 = nullptr;
@@ -1130,6 +1094,21 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
     if (o->precond == SHK_PRECOND_CHEBYSHEV) {
         if (o->cheb_degree < 1 || o->cheb_degree > kMaxChebDegree)
             return fail(c, SHK_BAD_ARG, "chebyshev_degree must be in [1, 32]");
+        if (o->cheb_nsteps < 2 || o->cheb_nsteps > kMaxChebSteps)
+            return fail(c, SHK_BAD_ARG, "chebyshev nsteps must be in [2, 64]");
+    }
+    // the whole solve in one persistent kernel where the grid's Krylov state fits on the chip
+    if (res_serves(c, o)) {
+        int rc = res_solve(c, o, make_cg_init(o, n, false, 0.0), ws ? ws : c->st.h);
+        if (rc) return rc;
+        if (deferred) {
+            *deferred = true;
+            return SHK_OK;
+        }
+        if ((rc = read_scalars(c))) return rc;
+        return collect_cg(c, o, st);
+    }
+    if (o->precond == SHK_PRECOND_CHEBYSHEV) {
         // _cg_precond! refreshes the bounds from this solve's rhs (src/linear_solver.jl:853-856)
         int rc = run_chebyshev_bounds(c, o->cheb_nsteps, c->rhs);
         if (rc) return rc;
@@ -1152,12 +1131,7 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
         c->launches++;
         if ((rc = check_launch(c, "cg finish"))) return rc;
         if ((rc = read_scalars(c))) return rc;
-        const CgDev &g = c->host_dev->cg;
-        if (g.fault) return fail(c, SHK_CUDA_ERROR, "a TMA tile copy did not complete (bounded wait ran out)");
-        s.niter = (long)g.iter;
-        s.status = g.status;
-        s.rnorm0 = g.rnorm0;
-        s.rnorm = g.rnorm;
+        if ((rc = collect_cg(c, o, &s))) return rc;
     } else if (o->precision == SHK_MIXED) {
         // Float32 stencil and CG with Float64 residual replacement.  The Float32 CG runs until its
         // recursive residual has dropped by inner_rtol; then its correction is folded into the
@@ -1252,11 +1226,8 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
     } else {
         return fail(c, SHK_BAD_ARG, "unknown precision");
     }
-    if ((o->precond == SHK_PRECOND_CHEBYSHEV)) {
-        if (o->precision != SHK_FP64) {
-            int rc = read_scalars(c);
-            if (rc) return rc;
-        }
+    if (o->precond == SHK_PRECOND_CHEBYSHEV && o->precision != SHK_FP64) {
+        if (int rc = read_scalars(c)) return rc;
         s.lambda_min = c->host_dev->cheb.lam_min;
         s.lambda_max = c->host_dev->cheb.lam_max;
         s.bounds_valid = c->host_dev->cheb.adopted;
