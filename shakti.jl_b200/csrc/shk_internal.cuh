@@ -163,6 +163,7 @@ struct Ctx {
     float mg_s2 = 1.0f;
     int mg_fused = 1;        // nu = 2 level kernels: 1 tile (default), 2 warp-marching, 0 per-sweep
     int mg_tma = 1;          // tile kernels stage through TMA copies where the level's pitch allows
+    bool mg_bottom2 = true;   // the bottom levels by k_mg_bottom (else the general one-block form)
     bool mg_cluster = false;  // the coarse levels on one thread-block cluster (measured slower; opt-in)
     bool mg_pair_x = true;    // the outer CG's x updated once per two iterations (bit-identical x)
     struct MgTma *mg_maps = nullptr;  // the levels' tensor maps (built on first use)
