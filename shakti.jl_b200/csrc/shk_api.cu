@@ -87,7 +87,9 @@ static int ctx_alloc(Ctx *c) {
         c->res_halo_bytes = std::max(c->res_halo_bytes, res_halo_bytes(P));
         vec_bytes = std::max(vec_bytes, res_vec_bytes(P));
     }
-    const size_t o_red = carve(c->res_red_bytes), o_halo = carve(c->res_halo_bytes), o_vec = carve(vec_bytes);
+    const size_t o_red = carve(c->res_red_bytes), o_halo = carve(c->res_halo_bytes),
+                 // the scratch vectors take the place of the general kernels' Krylov vectors
+                 o_vec = vec_bytes <= o_hprev - o_x ? o_x : carve(vec_bytes);
     size_t o_part = carve((size_t)kMaxRedValues * c->max_blocks * sizeof(double));
     size_t o_cnt = carve(64);
     size_t o_dev = carve(sizeof(DevScalars));

@@ -189,6 +189,7 @@ struct Ctx {
     cudaStream_t cap_stream = nullptr;  // capture only; nothing executes on it
     int graph_mode = 2;                 // 0 direct launches, 1 one graph per iteration, 2 device-side loop
     bool graphs_disabled = false;       // set when capture fails: direct launches from then on
+    long long loop_trip_launches = 0;   // kernels per trip of a device loop not yet accounted for
     bool loop_disabled = false;         // set when the device-loop graph cannot be built
     std::string err;
     bool assembled = false;
@@ -324,6 +325,5 @@ int mg_cg_matvec(Ctx *c, int par, const double *aP, const double *aE, const doub
                  const double *p_old, double *p_new, double *Ap, CgDev *cg, double eps_curv, bool *launched);
 int mg_apply_fused_update(Ctx *c, const double *r_in, double *r_out, double *x, const double *p, const double *Ap,
                           double *z, CgDev *cg, const double *p_prev = nullptr, int mode = 0, int pbuf = 0);
-int mg_catch_up(Ctx *c, double *x, CgDev *cg);
 
 } // namespace shk

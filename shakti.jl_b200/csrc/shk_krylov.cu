@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) k_matvec(int nx, int ny, const T *aP
 template <typename T, bool JAC>
 __device__ __forceinline__ void cg_init_body(Blk B, int nx, int ny, const T *aP, const T *aE, const T *aN,
                                              const double *x0, const T *b, T *r, T *x, CgDev *cg, double *partials,
-                                             unsigned int *counter, const uint8_t *fmask) {
+                                             unsigned int *counter, const uint8_t *fmask, const CgDev *start = nullptr) {
     Tiles Tl(nx, ny);
     double red[3] = {0.0, 0.0, 0.0};
     for (int t = B.id; t < Tl.ntiles; t += B.n) {
@@ -98,6 +98,7 @@ __device__ __forceinline__ void cg_init_body(Blk B, int nx, int ny, const T *aP,
     }
     double out[3];
     if (grid_reduce<3, false>(B, red, partials, counter, out) && threadIdx.x == 0) {
+        if (start) *cg = *start;
         if (JAC) cg_init_finish(cg, out[0], out[1], out[2]);
         else {
             cg->rr = out[1];    // parked: squared norms, consumed by the Chebyshev init pass
@@ -109,8 +110,9 @@ __device__ __forceinline__ void cg_init_body(Blk B, int nx, int ny, const T *aP,
 template <typename T, bool JAC>
 __global__ void __launch_bounds__(kThreads) k_cg_init(int nx, int ny, const T *aP, const T *aE, const T *aN,
                                                       const double *x0, const T *b, T *r, T *x, CgDev *cg,
-                                                      double *partials, unsigned int *counter, const uint8_t *fmask) {
-    cg_init_body<T, JAC>(grid_blk(), nx, ny, aP, aE, aN, x0, b, r, x, cg, partials, counter, fmask);
+                                                      double *partials, unsigned int *counter, const uint8_t *fmask,
+                                                      const __grid_constant__ CgDev start) {
+    cg_init_body<T, JAC>(grid_blk(), nx, ny, aP, aE, aN, x0, b, r, x, cg, partials, counter, fmask, &start);
 }
 
 // A: p_new = z + beta*p_old (p_new = z on the first iteration), Ap = A p_new, partial p'Ap.
@@ -371,6 +373,20 @@ __device__ __forceinline__ void cg_finish_body(Blk B, int n, const double *x, do
     for (int i = B.id * blockDim.x + threadIdx.x; i < n; i += B.n * blockDim.x) h[i] = x[i] + h[i];
 }
 __global__ void k_cg_finish(int n, const double *x, double *h) { cg_finish_body(grid_blk(), n, x, h); }
+// Multigrid form: h = x + x0 with the x update that the last iteration left pending (CgDev::x_pending;
+// the rounding of the single update).  One pass where the update and the addition took two (60 and
+// 66 us at 4096^2).
+__global__ void k_cg_finish_mg(int n, const double *x, const double *x0, double *h, const double *p0, const double *p1,
+                               const CgDev *cg) {
+    const int pend = cg->x_pending;
+    const double *p = pend == 1 ? p0 : p1;
+    const double a = cg->alpha;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double v = x[i];
+        if (pend) v = v + a * p[i];
+        h[i] = v + x0[i];
+    }
+}
 // h = x + x0 for a warm start x0 other than h
 __global__ void k_cg_finish_from(int n, const double *x, const double *x0, double *h) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) h[i] = x[i] + x0[i];
@@ -778,6 +794,11 @@ __global__ void k_cg_loop_cond(CgDev *cg, cudaGraphConditionalHandle h) {
     cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
+// The loop's condition at its start: a solve that its initial residual already satisfies runs no trip.
+__global__ void k_cg_loop_start(const CgDev *cg, cudaGraphConditionalHandle h) {
+    cudaGraphSetConditional(h, *(const volatile int *)&cg->done ? 0u : 1u);
+}
+
 static CgDev make_cg_init(const shk_cg_opts *o, long long n, bool inner, double inner_rtol) {
     CgDev g;
     memset(&g, 0, sizeof(g));
@@ -791,12 +812,22 @@ static CgDev make_cg_init(const shk_cg_opts *o, long long n, bool inner, double 
     return g;
 }
 
+// How a device-side loop ended, from the scalars read back after it.
+static int loop_ended(Ctx *c, const CgDev &g) {
+    c->launches += c->loop_trip_launches * (long long)g.trips;
+    c->loop_trip_launches = 0;
+    if (!g.done) return fail(c, SHK_CUDA_ERROR, "cg device loop reached its trip bound before stopping");
+    return SHK_OK;
+}
+
 // One preconditioned CG solve in precision T on system (aP, aE, aN), b -> x (correction from x0).
 // x0 (Float64, may be null) is the warm start used only for the initial residual.
+// With wait = false the device-side loop is left running: the caller reads the scalars after the work
+// it queues next, and collect_cg looks at how the loop ended.
 template <typename T>
 static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T *aP, const T *aE, const T *aN,
                    const double *x0, const T *b, T *x, T *r, T *z, T **p, T *Ap, T **cr, T **cp, long *iters_out,
-                   int p_parity = 0, const T *lapl = nullptr) {
+                   int p_parity = 0, const T *lapl = nullptr, bool wait = true) {
     const int nx = c->nx, ny = c->ny, n = nx * ny;
     const bool jac = o->precond == SHK_PRECOND_JACOBI;
     const bool mg = o->precond == SHK_PRECOND_MULTIGRID;
@@ -816,15 +847,14 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
             if (int rc0 = cg_tma_prepare(c)) return rc0;
     }
     cgh->trips = 0;
-    if (int rc0 = move_scalars(c, cgd, cgh, sizeof(CgDev), false)) return rc0;
     cudaError_t e = cudaSuccess;
     if (jac) {
         k_cg_init<T, true><<<c->grid_stencil, kThreads, 0, c->stream>>>(nx, ny, aP, aE, aN, x0, b, r, x, cgd, c->partials,
-                                                                       c->counter, c->mask8);
+                                                                       c->counter, c->mask8, *cgh);
         c->launches++;
     } else {
         k_cg_init<T, false><<<c->grid_stencil, kThreads, 0, c->stream>>>(nx, ny, aP, aE, aN, x0, b, r, x, cgd,
-                                                                        c->partials, c->counter, c->mask8);
+                                                                        c->partials, c->counter, c->mask8, *cgh);
         c->launches++;
         int prc = apply_precond(true);
         if (prc) return prc;
@@ -897,13 +927,6 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
         return SHK_OK;
     };
 
-    // a pending x update of the paired form, applied after the last iteration
-    auto catch_up = [&]() -> int {
-        if constexpr (std::is_same<T, double>::value) {
-            if (fuse_update && !jac && !lapl) return mg_catch_up(c, x, cgd);
-        }
-        return SHK_OK;
-    };
     // Graphs are keyed by everything that their kernel arguments depend on within one context.
     const long long key_base = ((long long)(lapl != nullptr) << 41) | ((long long)(sizeof(T) == 4) << 40) |
                                ((long long)o->precond << 32) | ((long long)deg << 8);
@@ -958,8 +981,14 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
                 np.conditional.handle = handle;
                 np.conditional.type = cudaGraphCondTypeWhile;
                 np.conditional.size = 1;
-                cudaGraphNode_t node;
-                ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+                cudaGraphNode_t node, begin;
+                size_t nodes = 1;
+                ok = capture(&graph, true, [&]() -> int {
+                         k_cg_loop_start<<<1, 1, 0, c->stream>>>(cgd, handle);
+                         return check_launch(c, "cg loop start");
+                     }) >= 0 &&
+                     cudaGraphGetNodes(graph, &begin, &nodes) == cudaSuccess && nodes == 1 &&
+                     cudaGraphAddNode(&node, graph, &begin, 1, &np) == cudaSuccess;
                 if (ok) {
                     cudaGraph_t body = np.conditional.phGraph_out[0];
                     per_trip = capture(&body, true, [&]() -> int {
@@ -984,15 +1013,13 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
             }
         }
         if (slot) {
+            e = cudaGraphLaunch(slot->exec, c->stream);
+            if (e != cudaSuccess) return check_cuda(c, e, "cg loop graph launch");
+            c->launches++;
+            c->loop_trip_launches = slot->launches;
+            if (!wait) return SHK_OK;
             if ((rc = read_cg_flags(c, cgh, cgd))) return rc;
-            if (!cgh->done) {
-                e = cudaGraphLaunch(slot->exec, c->stream);
-                if (e != cudaSuccess) return check_cuda(c, e, "cg loop graph launch");
-                if ((rc = read_cg_flags(c, cgh, cgd))) return rc;
-                c->launches += slot->launches * (long long)cgh->trips;
-                if (!cgh->done) return fail(c, SHK_CUDA_ERROR, "cg device loop reached its trip bound before stopping");
-            }
-            if ((rc = catch_up())) return rc;
+            if ((rc = loop_ended(c, *cgh))) return rc;
             if (iters_out) *iters_out = (long)cgh->iter;
             return SHK_OK;
         }
@@ -1044,7 +1071,6 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
         if (cgh->iter > cgh->itmax + 4 || enq > cgh->itmax + 2LL * batch_max + 8)
             return fail(c, SHK_CUDA_ERROR, "cg iteration accounting overran itmax");
     }
-    if ((rc = catch_up())) return rc;
     if (iters_out) *iters_out = (long)cgh->iter;
     return SHK_OK;
 }
@@ -1058,6 +1084,8 @@ int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
                                            ? "an exchange of the resident solve did not complete (bounded wait ran out)"
                                            : "a TMA tile copy did not complete (bounded wait ran out)");
     }
+    if (c->loop_trip_launches)
+        if (int rc = loop_ended(c, g)) return rc;
     memset(st, 0, sizeof(*st));
     st->niter = (long)g.iter;
     st->status = g.status;
@@ -1122,14 +1150,21 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
         // warm start: the head, or a one-shot caller-provided guess (shk_set_cg_warm_start)
         const double *x0 = ws ? ws : c->st.h;
         int rc = cg_core<double>(c, o, &c->dev->cg, cgh, c->aP, c->aE, c->aN, x0, c->rhs, c->x, c->r, c->z, c->p,
-                                 c->Ap, c->cr, c->cp, &it);
+                                 c->Ap, c->cr, c->cp, &it, 0, nullptr, deferred == nullptr);
         if (rc) return rc;
-        if (x0 == c->st.h)
+        if (o->precond == SHK_PRECOND_MULTIGRID)
+            k_cg_finish_mg<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, x0, c->st.h, c->p[0], c->p[1],
+                                                                        &c->dev->cg);
+        else if (x0 == c->st.h)
             k_cg_finish<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, c->st.h);
         else
             k_cg_finish_from<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, x0, c->st.h);
         c->launches++;
         if ((rc = check_launch(c, "cg finish"))) return rc;
+        if (deferred) {
+            *deferred = true;
+            return SHK_OK;
+        }
         if ((rc = read_scalars(c))) return rc;
         if ((rc = collect_cg(c, o, &s))) return rc;
     } else if (o->precision == SHK_MIXED) {
@@ -1484,7 +1519,7 @@ extern "C" SHK_API int shk_cg_solve_static(int nx, int ny, const double *aP, con
     init.first = 1;
     k_static_init<<<1, 32, 0, s>>>(cg, init, counter);
     k_cg_init<double, true><<<grid_stencil, kThreads, 0, s>>>(nx, ny, aP, aE, aN, x, rhs, r, xc, cg, partials, counter,
-                                                              nullptr);
+                                                              nullptr, init);
     if (cudaGetLastError() != cudaSuccess) return SHK_CUDA_ERROR;
     CgDev h;
     long long enq = 0;

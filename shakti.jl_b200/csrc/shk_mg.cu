@@ -189,6 +189,23 @@ __global__ void k_mg_coarsen_finish(int nxf, int nyf, int nxc, int nyc, const do
     coarsen_finish_cell(k, nxf, nyf, nxc, aEf, aNf, dPf, actf, omega, aEc, aNc, dPc, actc, fE, fN, fD, fW);
 }
 
+// The coarsening of every level of at most kRestCells cells by one block: a launch per level took 6 to
+// 8 us whatever its size, 47 us of a set-up at 256^2 for the levels from 64 x 64 down.
+constexpr int kRestCells = 4096;
+struct CoarsenLevels {
+    int n;  // levels, lv[0] the fine side of the first coarsening
+    MgLevel lv[kMgMaxLevels];
+};
+__global__ void __launch_bounds__(1024) k_mg_coarsen_rest(const __grid_constant__ CoarsenLevels C, double omega) {
+    for (int l = 0; l + 1 < C.n; l++) {
+        const MgLevel &f = C.lv[l], &g = C.lv[l + 1];
+        for (int k = threadIdx.x; k < g.nx * g.ny; k += blockDim.x)
+            coarsen_finish_cell(k, f.nx, f.ny, g.nx, f.aE64, f.aN64, f.dP64, f.act, omega, g.aE64, g.aN64, g.dP64, g.act,
+                                g.aE, g.aN, g.dP, g.wD);
+        __syncthreads();
+    }
+}
+
 // Float32 copies and the smoother's damped inverse diagonal wD = omega/aP with the Jacobi diagonal
 // aP = dP + the four couplings (identity rows: aP = 1, wD = 1).
 __device__ __forceinline__ void finish_level_cell(int k, int nx, const double *aE, const double *aN,
@@ -2165,6 +2182,14 @@ int mg_setup(Ctx *c) {
     for (int l = 0; l + 1 < c->mg_levels; l++) {
         const MgLevel &f = lv[l];
         MgLevel &g = lv[l + 1];
+        if (l > 0 && (long long)g.nx * g.ny <= kRestCells) {  // this level and all below it
+            CoarsenLevels C;
+            C.n = c->mg_levels - l;
+            for (int k = 0; k < C.n; k++) C.lv[k] = lv[l + k];
+            k_mg_coarsen_rest<<<1, 1024, 0, c->stream>>>(C, (double)c->mg_omega);
+            c->launches++;
+            break;
+        }
         if (l > 0) {  // coarsening and the coarse level's Float32 copies in one pass
             k_mg_coarsen_finish<<<mg_grid(c, (long long)g.nx * g.ny), kThreads, 0, c->stream>>>(
                 f.nx, f.ny, g.nx, g.ny, f.aE64, f.aN64, f.dP64, f.act, (double)c->mg_omega, g.aE64, g.aN64, g.dP64,
@@ -2612,23 +2637,6 @@ int cg_jac_matvec(Ctx *c, int par, const double *r, const double *p_old, double 
 // One iteration's x/r update fused into the V-cycle's first level-0 kernel (tile form, nu = 2):
 // r_new = r_in - alpha Ap into r_out, x += alpha p, then z = M^-1 r_new and the CG's r'z, r'r.
 bool mg_fuses_cg_update(const Ctx *c) { return marching(c) ? false : fused(c) && c->mg_levels > 1; }
-
-// After a solve whose last iteration was the first of a pair: x += alpha p for the pending p (the
-// rounding of the single update).  Returns at once when nothing is pending.
-__global__ void k_cg_catchup(long long n, double *x, const double *p0, const double *p1, const CgDev *cg) {
-    const int pend = cg->x_pending;
-    if (!pend) return;
-    const double *p = pend == 1 ? p0 : p1;
-    const double a = cg->alpha;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        x[i] = __dadd_rn(x[i], __dmul_rn(a, p[i]));
-}
-
-int mg_catch_up(Ctx *c, double *x, CgDev *cg) {
-    k_cg_catchup<<<c->num_sms * 8, 256, 0, c->stream>>>((long long)c->nx * c->ny, x, c->p[0], c->p[1], cg);
-    c->launches++;
-    return check_launch(c, "cg pending x update");
-}
 
 // mode / p_prev / pbuf: the paired x update of FusedB (mode 0: x updated every iteration); the
 // pairing needs the TMA-staged kernel, whose matvec records alpha_prev.
