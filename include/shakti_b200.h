@@ -318,6 +318,13 @@ SHK_API int shk_nn_mse(const float *Yf, const float *T, const float *wgt, float 
 SHK_API int shk_nn_adam(float *w, const float *g, float *m, float *v, void *wb, void *wt, long long n,
                         int Cout, int Cin, float lr, float b1, float b2, float eps, int step,
                         void *stream);
+/* shk_nn_adam on `count` tensors in one launch per 32 (host arrays of device pointers; wb[k], wt[k] may
+ * be NULL), and zeros in `count` tensors */
+SHK_API int shk_nn_adam_group(int count, float *const *w, const float *const *g, float *const *m,
+                              float *const *v, void *const *wb, void *const *wt, const long long *n,
+                              const int *cout, const int *cin, float lr, float b1, float b2, float eps,
+                              int step, void *stream);
+SHK_API int shk_nn_zero_group(int count, float *const *p, const long long *n, void *stream);
 SHK_API int shk_nn_wcast(const float *w, void *wb, void *wt, long long n, int Cout, int Cin,
                          void *stream);
 SHK_API int shk_nn_zero(float *p, long long n, void *stream);

@@ -73,6 +73,7 @@ class shk_ensemble_stats(C.Structure):
 # Every symbol include/shakti_b200.h declares, with (restype, argtypes).
 VP = C.c_void_p
 FP = C.POINTER(C.c_float)
+VPP = C.POINTER(VP)
 SIGNATURES = {
     "shk_version": (C.c_int, []),
     "shk_status_string": (C.c_char_p, [C.c_int]),
@@ -122,6 +123,9 @@ SIGNATURES = {
     "shk_nn_mse": (C.c_int, [FP, FP, FP, FP, FP, C.c_longlong, C.c_int, C.c_float, VP]),
     "shk_nn_adam": (C.c_int, [FP, FP, FP, FP, VP, VP, C.c_longlong, C.c_int, C.c_int, C.c_float, C.c_float,
                               C.c_float, C.c_float, C.c_int, VP]),
+    "shk_nn_adam_group": (C.c_int, [C.c_int, VPP, VPP, VPP, VPP, VPP, VPP, C.POINTER(C.c_longlong), C.POINTER(C.c_int),
+                                    C.POINTER(C.c_int), C.c_float, C.c_float, C.c_float, C.c_float, C.c_int, VP]),
+    "shk_nn_zero_group": (C.c_int, [C.c_int, VPP, C.POINTER(C.c_longlong), VP]),
     "shk_nn_wcast": (C.c_int, [FP, VP, VP, C.c_longlong, C.c_int, C.c_int, VP]),
     "shk_nn_zero": (C.c_int, [FP, C.c_longlong, VP]),
     "shk_nn_pack_state": (C.c_int, [C.POINTER(shk_state), C.c_int, C.c_int, C.c_int, C.c_int, FP, VP, VP]),

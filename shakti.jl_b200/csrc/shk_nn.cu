@@ -628,69 +628,88 @@ __global__ void __launch_bounds__(kHxThreads, 1) k_conv3x3_hx(const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------------
-// Weight gradient dW[tap, co, ci] += sum over a chunk of pixels of dY[p, co] X[p + off(tap), ci].
-// GEMM M = co (16 per block), N = ci (64 per block, 16 per warp), K = pixels (16 per step).  The
-// fragments gather pixel pairs (NHWC keeps channels, not pixels, contiguous), so they are built
-// from 16-bit loads.  grid = (pixel chunks, Cout/16 * ceil(Cin/64), 9).
+// Weight gradient dW[tap, co, ci] += sum over a chunk of pixels of dY[p, co] X[p + off(tap), ci]:
+// GEMM M = co, N = ci, K = pixels.  One block: kWgPx pixels, a 32 x 32 tile of (co, ci), one tap; four
+// warps of 16 x 16.  NHWC keeps channels contiguous, so both operands lie K-major-last: their tiles go to
+// shared memory as they are (16-byte asynchronous copies, zeros outside the image and past the
+// channels) and ldmatrix.trans forms the fragments.  All of a block's copies are in flight before its
+// only wait: at the sizes of a training batch (512 to 32768 pixels a layer) the kernel is bound by that
+// latency and by blocks in flight, not by the tensor cores, so the chunk is short (1152 blocks for 32
+// channels at 32768 pixels).  Rows are padded to 80 bytes: ldmatrix's 8 rows fall on different banks.
+// 8 to 14 us per layer (cold); a form with 1024-pixel chunks and fragments built from 16-bit global loads
+// took 70 to 120.
+// grid = (pixel chunks, ceil(Cout/32) * ceil(Cin/32), 9).  VEC: 16-byte aligned tensors (else 16-bit
+// loads).
 // ---------------------------------------------------------------------------------------------
-constexpr int kWgChunk = 1024;
+constexpr int kWgPx = 256, kWgTile = 32, kWgPitch = 40;
 
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const bf16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(su32(p)));
+}
+
+template <bool VEC>
 __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ dY,
                                                        float *__restrict__ dW, int N, int H, int W, int Cin,
                                                        int Cout) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    __shared__ __align__(16) bf16 sY[kWgPx * kWgPitch], sX[kWgPx * kWgPitch];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tap = blockIdx.z, dy = tap / 3 - 1, dx = tap % 3 - 1;
-    const int ntile_ci = (Cin + 63) / 64;
-    const int co0 = (blockIdx.y / ntile_ci) * 16, ci_blk = (blockIdx.y % ntile_ci) * 64;
-    const int ciw = ci_blk + warp * 16;  // this warp's 16 input channels (two n-tiles of 8)
-    if (ciw >= Cin) return;
-    const long long P = (long long)N * H * W;
-    const long long pbeg = (long long)blockIdx.x * kWgChunk, pend = min(P, pbeg + kWgChunk);
-    float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    const unsigned short *dYs = reinterpret_cast<const unsigned short *>(dY);
-    const unsigned short *Xs = reinterpret_cast<const unsigned short *>(X);
-    // source offset of pixel p shifted by the tap, or -1 outside the image
-    auto src = [&](long long p) -> long long {
-        if (p >= pend) return -1;
-        const long long hw = (long long)H * W;
-        const int n = (int)(p / hw), q = (int)(p % hw), y = q / W + dy, x = q % W + dx;
-        if (y < 0 || y >= H || x < 0 || x >= W) return -1;
-        return ((long long)n * H + y) * W + x;
+    const int tiles_ci = (Cin + kWgTile - 1) / kWgTile;
+    const int co0 = (blockIdx.y / tiles_ci) * kWgTile, ci0 = (blockIdx.y % tiles_ci) * kWgTile;
+    const long long hw = (long long)H * W, P = N * hw, p0 = (long long)blockIdx.x * kWgPx;
+    // the chunk's first pixel; later ones are counted on from it
+    const long long n0 = p0 / hw;
+    const int q0 = (int)(p0 % hw), y0 = q0 / W, x0 = q0 % W;
+    auto copy = [&](bf16 *dst, const bf16 *src, bool in) {
+        if (VEC) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(su32(dst)), "l"(src), "r"(in ? 16 : 0)
+                         : "memory");
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) dst[k] = in ? src[k] : __ushort_as_bfloat16(0);
+        }
     };
-    for (long long k0 = pbeg; k0 < pend; k0 += 16) {
-        const long long pk[4] = {k0 + 2 * t, k0 + 2 * t + 1, k0 + 2 * t + 8, k0 + 2 * t + 9};
-        unsigned short av[2][4];  // A rows g and g+8 (co), k columns pk[]
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const bool in = pk[i] < pend;
-            av[0][i] = in ? dYs[pk[i] * Cout + co0 + g] : (unsigned short)0;
-            av[1][i] = in ? dYs[pk[i] * Cout + co0 + g + 8] : (unsigned short)0;
-        }
-        uint32_t a[4] = {(uint32_t)av[0][0] | ((uint32_t)av[0][1] << 16), (uint32_t)av[1][0] | ((uint32_t)av[1][1] << 16),
-                         (uint32_t)av[0][2] | ((uint32_t)av[0][3] << 16), (uint32_t)av[1][2] | ((uint32_t)av[1][3] << 16)};
-        long long s[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) s[i] = src(pk[i]);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int ci = ciw + j * 8 + g;
-            unsigned short bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) bv[i] = (s[i] >= 0 && ci < Cin) ? Xs[s[i] * Cin + ci] : (unsigned short)0;
-            uint32_t b[2] = {(uint32_t)bv[0] | ((uint32_t)bv[1] << 16), (uint32_t)bv[2] | ((uint32_t)bv[3] << 16)};
-            mma_bf16(acc[j], a, b);
-        }
+    for (int i = tid; i < kWgPx * (kWgTile / 8); i += 128) {
+        const int px = i / (kWgTile / 8), c = (i % (kWgTile / 8)) * 8;
+        const long long p = p0 + px;
+        const int xs = x0 + px, ys = y0 + xs / W, sx = xs % W + dx, sy = ys % H + dy;
+        const bool iny = p < P && co0 + c < Cout;
+        copy(sY + px * kWgPitch + c, iny ? dY + p * Cout + co0 + c : dY, iny);
+        const bool inx = p < P && ci0 + c < Cin && sx >= 0 && sx < W && sy >= 0 && sy < H;
+        const long long q = ((n0 + ys / H) * H + sy) * W + sx;
+        copy(sX + px * kWgPitch + c, inx ? X + q * Cin + ci0 + c : X, inx);
     }
+    if (VEC) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int m0 = (warp & 1) * 16, c0 = (warp >> 1) * 16;  // this warp's 16 x 16 of the tile
+    if (co0 + m0 >= Cout || ci0 + c0 >= Cin) return;
+    const int r = lane & 7, mat = lane >> 3;
+    // matrices 0..3 of A: (k, m) = (0, 0), (0, 8), (8, 0), (8, 8); of B: (k, n) = (0, 0), (8, 0), (0, 8), (8, 8)
+    const bf16 *pa = sY + ((mat >> 1) * 8 + r) * kWgPitch + m0 + (mat & 1) * 8;
+    const bf16 *pb = sX + ((mat & 1) * 8 + r) * kWgPitch + c0 + (mat >> 1) * 8;
+    float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+#pragma unroll 4
+    for (int k = 0; k < kWgPx; k += 16) {
+        uint32_t a[4], b[4];
+        ldmatrix_x4_trans(a, pa + k * kWgPitch);
+        ldmatrix_x4_trans(b, pb + k * kWgPitch);
+        const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+        mma_bf16(acc[0], a, b0);
+        mma_bf16(acc[1], a, b1);
+    }
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        const int ci = ciw + j * 8 + 2 * t;
+        const int ci = ci0 + c0 + j * 8 + 2 * t;
         if (ci >= Cin) continue;
-        float *w0 = dW + ((long long)tap * Cout + co0 + g) * Cin + ci;
-        float *w1 = dW + ((long long)tap * Cout + co0 + g + 8) * Cin + ci;
-        atomicAdd(w0, acc[j][0]);
-        atomicAdd(w0 + 1, acc[j][1]);
-        atomicAdd(w1, acc[j][2]);
-        atomicAdd(w1 + 1, acc[j][3]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float *w = dW + ((long long)tap * Cout + co0 + m0 + g + 8 * h) * Cin + ci;
+            atomicAdd(w, acc[j][2 * h]);
+            atomicAdd(w + 1, acc[j][2 * h + 1]);
+        }
     }
 }
 
@@ -700,18 +719,44 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const bf16 *__restrict__ 
 #define NN_GSTRIDE(i, n) \
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (n); i += (long long)gridDim.x * blockDim.x)
 
-// dYm = dY * (Y > 0) (ReLU; relu == 0: identity) in BF16; db[c] += sum of dYm over pixels.
+// dYm = dY * (Y > 0) (ReLU; relu == 0: identity) in BF16; db[c] += sum of dYm over pixels.  V
+// consecutive channels per thread, the same ones in every step (the grid's stride is a multiple of C
+// where C is a power of two), so their sums stay in registers until the end; other C take an atomic on
+// shared memory per element.  The grid is small on purpose: with 2048 blocks the last step, one
+// global atomic per block and channel on the same C addresses, took 10 of the kernel's 12 us.
+template <int V>
 __global__ void k_relu_grad(const float *__restrict__ dY, const bf16 *__restrict__ Y, bf16 *__restrict__ dYm,
                             float *__restrict__ db, long long P, int C, int relu) {
     extern __shared__ float sdb[];
     for (int c = threadIdx.x; c < C; c += blockDim.x) sdb[c] = 0.0f;
     __syncthreads();
-    NN_GSTRIDE(i, P * C) {
-        float v = dY[i];
-        if (relu && !(__bfloat162float(Y[i]) > 0.0f)) v = 0.0f;
-        dYm[i] = __float2bfloat16(v);
-        if (db) atomicAdd(&sdb[i % C], v);
+    const bool fixed = ((long long)gridDim.x * blockDim.x * V) % C == 0;
+    const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * V;
+    float sum[V] = {};
+    for (long long i = first; i < P * C; i += (long long)gridDim.x * blockDim.x * V) {
+        float v[V];
+        bf16 y[V], o[V];
+        if constexpr (V == 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(dY + i);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            if (relu) *reinterpret_cast<uint2 *>(y) = *reinterpret_cast<const uint2 *>(Y + i);
+        } else {
+            v[0] = dY[i];
+            if (relu) y[0] = Y[i];
+        }
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+            if (relu && !(__bfloat162float(y[k]) > 0.0f)) v[k] = 0.0f;
+            o[k] = __float2bfloat16(v[k]);
+            if (fixed) sum[k] += v[k];
+            else if (db) atomicAdd(&sdb[(i + k) % C], v[k]);
+        }
+        if constexpr (V == 4) *reinterpret_cast<uint2 *>(dYm + i) = *reinterpret_cast<const uint2 *>(o);
+        else dYm[i] = o[0];
     }
+    if (db && fixed && first < P * C)
+#pragma unroll
+        for (int k = 0; k < V; k++) atomicAdd(&sdb[(int)((first + k) % C)], sum[k]);
     __syncthreads();
     if (db)
         for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&db[c], sdb[c]);
@@ -798,27 +843,68 @@ __global__ void k_mse(const float *__restrict__ Yf, const float *__restrict__ T,
 // Adam (bias-corrected), Float32 master weights; refreshes the BF16 copy and, when WT is given,
 // the per-tap transposed copy used by the input-gradient convolution (layout [9][Cout][Cin] ->
 // [9][Cin][Cout]).
+__device__ __forceinline__ void adam_element(long long i, float *w, const float *g, float *m, float *v, bf16 *wb, bf16 *wt,
+                                             int Cout, int Cin, float lr, float b1, float b2, float eps, float c1,
+                                             float c2) {
+    float gi = g[i];
+    float mi = b1 * m[i] + (1.0f - b1) * gi;
+    float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i] = wi;
+    const bf16 b = __float2bfloat16(wi);
+    if (wb) wb[i] = b;
+    if (wt) {
+        const long long per = (long long)Cout * Cin;
+        const long long tap = i / per, r = i % per;
+        const int co = (int)(r / Cin), ci = (int)(r % Cin);
+        wt[tap * per + (long long)ci * Cout + co] = b;
+    }
+}
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                        bf16 *__restrict__ wb, bf16 *__restrict__ wt, long long n, int Cout, int Cin, float lr,
                        float b1, float b2, float eps, float c1, float c2) {
-    NN_GSTRIDE(i, n) {
-        float gi = g[i];
-        float mi = b1 * m[i] + (1.0f - b1) * gi;
-        float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[i] = wi;
-        const bf16 b = __float2bfloat16(wi);
-        if (wb) wb[i] = b;
-        if (wt) {
-            const long long per = (long long)Cout * Cin;
-            const long long tap = i / per, r = i % per;
-            const int co = (int)(r / Cin), ci = (int)(r % Cin);
-            wt[tap * per + (long long)ci * Cout + co] = b;
-        }
+    NN_GSTRIDE(i, n) adam_element(i, w, g, m, v, wb, wt, Cout, Cin, lr, b1, b2, eps, c1, c2);
+}
+// Every tensor of a group in one launch: a network's 30 tensors of 16 to 590,000 elements took a launch
+// of 3 to 12 us each, most of them for a few blocks' work.  Block k belongs to the tensor whose range of
+// blocks it falls in.
+constexpr int kGroup = 32, kGroupChunk = 1024;
+struct TensorGroup {
+    int count, block0[kGroup + 1];
+    long long n[kGroup];
+    float *w[kGroup], *m[kGroup], *v[kGroup];
+    const float *g[kGroup];
+    bf16 *wb[kGroup], *wt[kGroup];
+    int cout[kGroup], cin[kGroup];
+};
+__device__ __forceinline__ int group_of(const TensorGroup &G, int block) {
+    int t = 0;
+    while (t + 1 < G.count && block >= G.block0[t + 1]) t++;
+    return t;
+}
+__global__ void __launch_bounds__(256) k_adam_group(const __grid_constant__ TensorGroup G, float lr, float b1, float b2,
+                                                    float eps, float c1, float c2) {
+    const int t = group_of(G, blockIdx.x);
+    const long long i0 = (long long)(blockIdx.x - G.block0[t]) * kGroupChunk;
+#pragma unroll
+    for (int k = 0; k < kGroupChunk; k += 256) {
+        const long long i = i0 + k + threadIdx.x;
+        if (i < G.n[t])
+            adam_element(i, G.w[t], G.g[t], G.m[t], G.v[t], G.wb[t], G.wt[t], G.cout[t], G.cin[t], lr, b1, b2, eps, c1, c2);
     }
 }
+__global__ void __launch_bounds__(256) k_zero_group(const __grid_constant__ TensorGroup G) {
+    const int t = group_of(G, blockIdx.x);
+    const long long i0 = (long long)(blockIdx.x - G.block0[t]) * kGroupChunk;
+#pragma unroll
+    for (int k = 0; k < kGroupChunk; k += 256) {
+        const long long i = i0 + k + threadIdx.x;
+        if (i < G.n[t]) G.w[t][i] = 0.0f;
+    }
+}
+
 // BF16 copy and per-tap transpose of a weight tensor (no update)
 __global__ void k_wcast(const float *__restrict__ w, bf16 *__restrict__ wb, bf16 *__restrict__ wt, long long n,
                         int Cout, int Cin) {
@@ -870,6 +956,28 @@ __global__ void k_apply_increment(const float *__restrict__ Yf, int C, int nx, i
 static int grid_for(long long n) {
     long long b = (n + 255) / 256;
     return (int)(b < 1 ? 1 : (b > 148 * 16 ? 148 * 16 : b));
+}
+
+// The tensors of a group, kGroup at a time; launch(first tensor's group, blocks).
+template <typename Fill, typename Launch>
+static int for_groups(int count, const long long *n, Fill fill, Launch launch) {
+    if (count < 0 || (count && !n)) return SHK_BAD_ARG;
+    for (int t0 = 0; t0 < count; t0 += kGroup) {
+        TensorGroup G = {};
+        long long blocks = 0;
+        G.count = count - t0 < kGroup ? count - t0 : kGroup;
+        for (int k = 0; k < G.count; k++) {
+            if (n[t0 + k] < 0) return SHK_BAD_ARG;
+            G.block0[k] = (int)blocks;
+            G.n[k] = n[t0 + k];
+            blocks += (n[t0 + k] + kGroupChunk - 1) / kGroupChunk;
+            if (blocks > 0x7fffffff || !fill(G, k, t0 + k)) return SHK_BAD_ARG;
+        }
+        G.block0[G.count] = (int)blocks;
+        if (blocks) launch(G, (int)blocks);
+        if (cudaGetLastError() != cudaSuccess) return SHK_CUDA_ERROR;
+    }
+    return SHK_OK;
 }
 
 } // namespace nn
@@ -1043,17 +1151,29 @@ SHK_API int shk_nn_conv3x3_wgrad(const void *X, const void *dY, float *dW, int N
                                  void *stream) {
     if (!X || !dY || !dW || Cin % 8 || Cout % 16) return SHK_BAD_ARG;
     const long long P = (long long)N * H * W;
-    dim3 grid((unsigned)((P + kWgChunk - 1) / kWgChunk), (unsigned)((Cout / 16) * ((Cin + 63) / 64)), 9);
-    k_conv3x3_wgrad<<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W, Cin,
-                                                            Cout);
+    dim3 grid((unsigned)((P + kWgPx - 1) / kWgPx),
+              (unsigned)(((Cout + kWgTile - 1) / kWgTile) * ((Cin + kWgTile - 1) / kWgTile)), 9);
+    if ((((uintptr_t)X | (uintptr_t)dY) & 15) == 0)
+        k_conv3x3_wgrad<true><<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W,
+                                                                      Cin, Cout);
+    else
+        k_conv3x3_wgrad<false><<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W,
+                                                                       Cin, Cout);
     return cudaGetLastError() == cudaSuccess ? SHK_OK : SHK_CUDA_ERROR;
 }
 
 SHK_API int shk_nn_relu_grad(const float *dY, const void *Y, void *dYm, float *db, long long P, int C, int relu,
                              void *stream) {
     if (C < 1 || C > 4096) return SHK_BAD_ARG;
-    k_relu_grad<<<grid_for(P * C), 256, C * sizeof(float), (cudaStream_t)stream>>>(dY, (const bf16 *)Y, (bf16 *)dYm,
-                                                                                   db, P, C, relu);
+    const bool vec = C % 4 == 0 && (((uintptr_t)dY & 15) | ((uintptr_t)Y & 7) | ((uintptr_t)dYm & 7)) == 0;
+    const long long blocks = (P * C + 256 * 4 - 1) / (256 * 4);
+    const int grid = (int)(blocks < 1 ? 1 : (blocks > 148 * 2 ? 148 * 2 : blocks));
+    if (vec)
+        k_relu_grad<4><<<grid, 256, C * sizeof(float), (cudaStream_t)stream>>>(dY, (const bf16 *)Y, (bf16 *)dYm, db, P,
+                                                                               C, relu);
+    else
+        k_relu_grad<1><<<grid, 256, C * sizeof(float), (cudaStream_t)stream>>>(dY, (const bf16 *)Y, (bf16 *)dYm, db, P,
+                                                                               C, relu);
     return cudaGetLastError() == cudaSuccess ? SHK_OK : SHK_CUDA_ERROR;
 }
 
@@ -1099,6 +1219,31 @@ SHK_API int shk_nn_adam(float *w, const float *g, float *m, float *v, void *wb, 
     k_adam<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(w, g, m, v, (bf16 *)wb, (bf16 *)wt, n, Cout, Cin, lr, b1, b2,
                                                           eps, c1, c2);
     return cudaGetLastError() == cudaSuccess ? SHK_OK : SHK_CUDA_ERROR;
+}
+
+SHK_API int shk_nn_adam_group(int count, float *const *w, const float *const *g, float *const *m, float *const *v,
+                              void *const *wb, void *const *wt, const long long *n, const int *cout, const int *cin,
+                              float lr, float b1, float b2, float eps, int step, void *stream) {
+    if (step < 1 || (count > 0 && (!w || !g || !m || !v || !wb || !wt || !cout || !cin))) return SHK_BAD_ARG;
+    const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
+    return for_groups(
+        count, n,
+        [&](TensorGroup &G, int k, int t) {
+            G.w[k] = w[t], G.g[k] = g[t], G.m[k] = m[t], G.v[k] = v[t];
+            G.wb[k] = (bf16 *)wb[t], G.wt[k] = (bf16 *)wt[t];
+            G.cout[k] = cout[t], G.cin[k] = cin[t];
+            return w[t] && g[t] && m[t] && v[t];
+        },
+        [&](const TensorGroup &G, int blocks) {
+            k_adam_group<<<blocks, 256, 0, (cudaStream_t)stream>>>(G, lr, b1, b2, eps, c1, c2);
+        });
+}
+
+SHK_API int shk_nn_zero_group(int count, float *const *p, const long long *n, void *stream) {
+    if (count > 0 && !p) return SHK_BAD_ARG;
+    return for_groups(
+        count, n, [&](TensorGroup &G, int k, int t) { return (G.w[k] = p[t]) != nullptr; },
+        [&](const TensorGroup &G, int blocks) { k_zero_group<<<blocks, 256, 0, (cudaStream_t)stream>>>(G); });
 }
 
 SHK_API int shk_nn_wcast(const float *w, void *wb, void *wt, long long n, int Cout, int Cin, void *stream) {

@@ -40,6 +40,14 @@ def _fp(t):
     return C.cast(C.c_void_p(t.data_ptr()), C.POINTER(C.c_float)) if t is not None else None
 
 
+def _ptrs(ts):
+    return (C.c_void_p * len(ts))(*[None if t is None else t.data_ptr() for t in ts])
+
+
+def _sizes(ts):
+    return (C.c_longlong * len(ts))(*[t.numel() for t in ts])
+
+
 class WarmStartNet:
     def __init__(self, seed: int = 0):
         import torch
@@ -161,10 +169,8 @@ class WarmStartNet:
         A = self._acts
         N, H, W, _ = A["x0"].shape
         f32 = self.torch.float32
-        for name, *_ in LAYERS:
-            p = self.P[name]
-            self._chk(self.L.shk_nn_zero(_fp(p["gw"]), p["gw"].numel(), self._s()), "zero")
-            self._chk(self.L.shk_nn_zero(_fp(p["gb"]), p["gb"].numel(), self._s()), "zero")
+        g = [self.P[name][k] for name, *_ in LAYERS for k in ("gw", "gb")]
+        self._chk(self.L.shk_nn_zero_group(len(g), _ptrs(g), _sizes(g), self._s()), "zero")
         d = self._layer_back("head", A["d0"], dY, None, N, H, W)
         hs = [(H, W), (H // 2, W // 2), (H // 4, W // 4), (H // 8, W // 8)]
         ds = {}
@@ -205,13 +211,15 @@ class WarmStartNet:
 
     def adam_step(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step_no += 1
-        for name, cin, cout, _ in LAYERS:
-            p = self.P[name]
-            self._chk(self.L.shk_nn_adam(_fp(p["w"]), _fp(p["gw"]), _fp(p["mw"]), _fp(p["vw"]), _p(p["wb"]),
-                                         _p(p["wt"]), p["w"].numel(), cout, cin, lr, b1, b2, eps, self.step_no,
-                                         self._s()), "adam")
-            self._chk(self.L.shk_nn_adam(_fp(p["b"]), _fp(p["gb"]), _fp(p["mb"]), _fp(p["vb"]), None, None,
-                                         p["b"].numel(), cout, 1, lr, b1, b2, eps, self.step_no, self._s()), "adam")
+        P = [self.P[name] for name, *_ in LAYERS]
+        w = [p[k] for p in P for k in ("w", "b")]
+        g, m, v = ([p[c + k] for p in P for k in ("w", "b")] for c in "gmv")
+        wb, wt = ([t for p in P for t in (p[k], None)] for k in ("wb", "wt"))
+        n = len(w)
+        cout = (C.c_int * n)(*[p["cout"] for p in P for _ in "wb"])
+        cin = (C.c_int * n)(*[c for p in P for c in (p["cin"], 1)])
+        self._chk(self.L.shk_nn_adam_group(n, _ptrs(w), _ptrs(g), _ptrs(m), _ptrs(v), _ptrs(wb), _ptrs(wt), _sizes(w),
+                                           cout, cin, lr, b1, b2, eps, self.step_no, self._s()), "adam")
 
     def train(self, X, T, M, steps: int, batch: int = 32, lr: float = 1e-3, seed: int = 0):
         """Adam on random mini-batches of the pairs (X [S,H,W,16] BF16, T/M [S,H,W] Float32)."""
