@@ -49,6 +49,10 @@ static void derive_params(Ctx *c) {
     P.dy = c->dy;
     P.dx2 = c->dx * c->dx;
     P.dy2 = c->dy * c->dy;
+    P.dx_inv = 1.0 / c->dx;
+    P.dy_inv = 1.0 / c->dy;
+    P.nu2x12 = 12 * (p.nu * p.nu);
+    P.nu2x12_inv = 1.0 / P.nu2x12;
 }
 
 static int ctx_alloc(Ctx *c) {

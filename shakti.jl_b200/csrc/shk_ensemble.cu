@@ -127,7 +127,6 @@ static int echeck(Ens *e, cudaError_t r, const char *what) {
     return efail(e, SHK_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(r));
 }
 
-static int tiles_of(int nx, int ny) { return ((nx + kTX - 1) / kTX) * ((ny + kTY - 1) / kTY); }
 static int march_blocks_of(int nx, int ny, int th) { return ((nx + kMarchX - 1) / kMarchX) * ((ny + th - 1) / th); }
 
 // Per-instance block counts of each family, the block -> instance tables, and the descriptors.
@@ -141,7 +140,7 @@ static int ens_layout(Ens *e) {
         // flat_grid in shk_krylov.cu)
         int nb[EF_N];
         nb[EF_STENCIL] = c->grid_stencil;
-        nb[EF_TAIL] = std::max(1, std::min(tiles_of(I.nx, I.ny), c->num_sms * kTailBlocksPerSm));
+        nb[EF_TAIL] = tail_blocks(I.nx, I.ny, c->num_sms);
         nb[EF_MARCH] = march_blocks_of(I.nx, I.ny, I.march_th);
         nb[EF_STREAM] = (int)std::max(1LL, std::min((long long)c->num_sms * 8, (n + 1023) / 1024));
         nb[EF_FLAT] = (int)std::max(1LL, std::min((long long)c->grid_stencil, (n + kThreads - 1) / kThreads));

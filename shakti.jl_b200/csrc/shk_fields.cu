@@ -149,7 +149,7 @@ struct FaceOut {
 
 __device__ __forceinline__ void q_re(const Params &P, double bf, double grad, double &q, double &re) {
     double G = fabs(grad);
-    double D = (bf * bf * bf * P.g * G) / (12 * (P.nu * P.nu));
+    double D = quotient_any(bf * bf * bf * P.g * G, P.nu2x12, P.nu2x12_inv);
     double R = 2 * D / (1 + sqrt(1 + 4 * P.omega * D));
     re = R;
     q = -jl_sign(grad) * P.nu * R;
@@ -161,6 +161,8 @@ __device__ __forceinline__ double taub_face(const Params &P, const Sliding &L, d
     if (L.kind == SHK_SLIDING_LINEAR) return Cf * Nf * ub;
     if (!(abs_v > 0)) return 0.0;
     double denom = (L.kind == SHK_SLIDING_REG_COULOMB_V0) ? L.v0 : jl_pow(fabs(Nf), P.n, P.n_int) * lf;
+    // no sliding across this face: the drag is 0 (with its sign), whatever the root below
+    if (ub == 0.0 && abs_v < INFINITY && denom == denom) return Nf * Cf * ub;
     // x^(1/n): for n = 3, cbrt (a fraction of pow's cost; it differs from pow(x, 1/3.0) by at most
     // about an ulp, within the tolerance the parity tests hold the pow-dependent fields to)
     const double ratio = abs_v / (abs_v + denom);
@@ -172,49 +174,62 @@ struct CellQ {
     double h, pw, N, lam, aub;
 };
 
+// What a cell's CellQ is formed from, as loaded: h, zb, po (FROM_H) or h, pw, N.
+struct CellRaw {
+    double a, b, c, lam, aub;
+    uint8_t m;
+};
 template <bool FROM_H>
-__device__ __forceinline__ CellQ load_cell(const Params &P, const shk_state &s, const uint8_t *m8, size_t c) {
+__device__ __forceinline__ CellRaw load_cell(const shk_state &s, const uint8_t *m8, unsigned c) {
+    CellRaw r;
+    r.a = s.h[c];
+    r.b = FROM_H ? s.zb[c] : s.pw[c];
+    r.c = FROM_H ? s.po[c] : s.N[c];
+    r.lam = s.lambda[c];
+    r.aub = s.abs_ub[c];
+    r.m = FROM_H ? m8[c] : 0;
+    return r;
+}
+template <bool FROM_H>
+__device__ __forceinline__ CellQ make_cell(const Params &P, const CellRaw &r) {
     CellQ q;
+    q.h = r.a;
     if (FROM_H) {
-        q.h = s.h[c];
-        q.pw = P.rho_w * P.g * (q.h - s.zb[c]);
-        double d = s.po[c] - q.pw;
-        q.N = (m8[c] == M_GROUNDED) ? d : copysign(0.0, d);
+        q.pw = P.rho_w * P.g * (q.h - r.b);
+        const double d = r.c - q.pw;
+        q.N = (r.m == M_GROUNDED) ? d : copysign(0.0, d);
     } else {
-        q.h = s.h[c];
-        q.pw = s.pw[c];
-        q.N = s.N[c];
+        q.pw = r.b;
+        q.N = r.c;
     }
-    q.lam = s.lambda[c];
-    q.aub = s.abs_ub[c];
+    q.lam = r.lam;
+    q.aub = r.aub;
     return q;
 }
 
-// x- (dir 0) or y-face (dir 1) between cells a (west/south) and b (east/north); a or b may be absent
+// A face's own inputs.
+struct FaceRaw {
+    double valid, b, ub;
+};
+
+// x- (DIR 0) or y-face (DIR 1) between cells a (west/south) and b (east/north); a or b may be absent
 // at the domain edge (edge face: gradients read from memory, taub uses the one adjacent cell).
-template <bool FROM_H>
-__device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const shk_state &s, int dir,
-                                        size_t fi, bool interior, const CellQ &a, const CellQ &b,
-                                        const CellQ &edge_cell) {
+template <bool FROM_H, int DIR>
+__device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const shk_state &s, unsigned fi, bool interior, const CellQ &a, const CellQ &b, const CellQ &edge_cell,
+                                        const FaceRaw &r) {
     FaceOut o;
-    const double *dhf = dir == 0 ? s.dhdx : s.dhdy;
-    const double *dpwf = dir == 0 ? s.dpwdx : s.dpwdy;
-    const double *valid = dir == 0 ? s.valid_x : s.valid_y;
-    const double *bface = dir == 0 ? s.b_x : s.b_y;
-    const double *ubf = dir == 0 ? s.ub_x : s.ub_y;
-    const double dd = dir == 0 ? P.dx : P.dy;
     if (interior && FROM_H) {
-        double v = valid[fi];
-        o.dh = ((b.h - a.h) / dd) * v;
-        o.dpw = ((b.pw - a.pw) / dd) * v;
+        const double dd = DIR == 0 ? P.dx : P.dy, inv = DIR == 0 ? P.dx_inv : P.dy_inv;
+        o.dh = quotient_any(b.h - a.h, dd, inv) * r.valid;
+        o.dpw = quotient_any(b.pw - a.pw, dd, inv) * r.valid;
     } else {
-        o.dh = dhf[fi];
-        o.dpw = dpwf[fi];
+        o.dh = (DIR == 0 ? s.dhdx : s.dhdy)[fi];
+        o.dpw = (DIR == 0 ? s.dpwdx : s.dpwdy)[fi];
     }
-    q_re(P, bface[fi], o.dh, o.q, o.re);
-    o.ub = ubf[fi];
+    q_re(P, r.b, o.dh, o.q, o.re);
+    o.ub = r.ub;
     if (L.kind == SHK_SLIDING_PRESCRIBED) {
-        o.taub = (dir == 0 ? s.taub_x : s.taub_y)[fi];
+        o.taub = (DIR == 0 ? s.taub_x : s.taub_y)[fi];
     } else {
         double Nf, lf, av;
         if (interior) {
@@ -226,7 +241,7 @@ __device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const
             lf = edge_cell.lam;
             av = edge_cell.aub;
         }
-        double Cf = (L.kind == SHK_SLIDING_REG_COULOMB) ? L.C : (dir == 0 ? L.Cx : L.Cy)[fi];
+        const double Cf = (L.kind == SHK_SLIDING_REG_COULOMB) ? L.C : (DIR == 0 ? L.Cx : L.Cy)[fi];
         o.taub = taub_face(P, L, Nf, lf, av, o.ub, Cf);
     }
     return o;
@@ -238,120 +253,141 @@ __device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const
 // plus the Picard check maxima max|h - h_prev| and max|h| (src/elliptic_solver.jl:162-163).
 // FROM_H = false is the initial-condition variant: pw, N and the gradients are taken as set.
 //
-// One 32 x 8 tile per block iteration, one thread per cell: (1) the tile's cells and a one-cell
-// halo (no corners) are loaded to shared memory with pw and N formed from h; (2) each of the
-// tile's 33 x 8 x-faces and 32 x 9 y-faces is computed once (q, Re, taub from the reference's
-// face formulas), the faces the tile owns are written, and the products the cells need
-// (Re, ub*taub, q*dh, q*dpw) stay in shared memory; (3) each cell sums its four faces.
+// A warp marches up a strip of 30 columns (lanes 1..30; lanes 0 and 31 hold the columns beside it).  Row by
+// row it forms the row's west faces from its cells (a lane's west cell by shuffle; its east face is the
+// next lane's west face) and the north faces from the row above, which the next row takes as its south
+// faces: no shared memory, no block barrier, every face computed once but for the strips' edges (6 %,
+// and one row of faces per strip).  The next row's 14 inputs are requested before the current row is
+// computed, so 16 warps per SM keep 45 KB of loads in flight.  The strips' height makes one wave of the
+// resident warps.
+// 257 B per cell: 344 us at 2501 x 1803 and 1240 us at 4096^2 (53 % of the copy rate), where the form
+// before it (32 x 8 tiles, faces through shared memory, three waits per tile) took 389 and 1302.  Bound
+// by latency: about 1000 instructions a row, a fifth of them Float64, in chains that the branches
+// inside divides, square roots and the cube root keep from overlapping, on 16 warps an SM (12 warps:
+// 399 us at 2501 x 1803; 20 with spills: 491; without the prefetch and 24 warps: 367).
 // ---------------------------------------------------------------------------------------------
-constexpr int kTailW = kTX, kTailH = kTY;           // cells per tile
-// 288 threads: the tile's 552 faces take two rounds (with 256 threads the third round would keep
-// only 40 threads busy while the rest waited at the barrier)
-constexpr int kTailThreads = 288;
-constexpr int kTailHW = kTailW + 2, kTailHH = kTailH + 2; // with the halo
-constexpr int kTailXF = (kTailW + 1) * kTailH;      // x-faces of a tile
-constexpr int kTailYF = kTailW * (kTailH + 1);      // y-faces of a tile
+constexpr int kTailCols = 30;  // output columns of a warp
 
-struct FaceSm {
+// What a cell needs of a face.
+struct FaceSums {
     double re, ut, qd, qp;  // Re, ub*taub, q*dh, q*dpw
 };
+__device__ __forceinline__ FaceSums face_sums(const FaceOut &o) {
+    return FaceSums{o.re, o.ub * o.taub, o.q * o.dh, o.q * o.dpw};
+}
 
 template <bool FROM_H, bool CHECK>
 __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P, const Sliding &L,
                                           const shk_state &s, const uint8_t *__restrict__ m8,
                                           const double *__restrict__ h_prev, double *partials, unsigned int *counter,
                                           PicDev *pic) {
-    __shared__ CellQ cq[kTailHH][kTailHW];
-    __shared__ FaceSm fx[kTailXF], fy[kTailYF];
-    const int tiles_x = (nx + kTailW - 1) / kTailW, ntiles = tiles_x * ((ny + kTailH - 1) / kTailH);
-    const int tid = threadIdx.x, tx = tid % kTailW, ty = tid / kTailW;
+    const int lane = threadIdx.x & 31, warps = B.n * (kTailThreads / 32);
+    const int nsx = (nx + kTailCols - 1) / kTailCols, per = max(1, warps / nsx), th = (ny + per - 1) / per,
+              strips = nsx * ((ny + th - 1) / th);
     double red[2] = {0.0, 0.0};
-    for (int t = B.id; t < ntiles; t += B.n) {
-        const int x0 = (t % tiles_x) * kTailW, y0 = (t / tiles_x) * kTailH;
-        // (1) cells of the tile and its halo
-        for (int k = tid; k < kTailHH * kTailHW; k += kTailThreads) {
-            const int hx = k % kTailHW, hy = k / kTailHW, ix = x0 - 1 + hx, iy = y0 - 1 + hy;
-            const bool corner = (hx == 0 || hx == kTailHW - 1) && (hy == 0 || hy == kTailHH - 1);
-            if (corner || ix < 0 || ix >= nx || iy < 0 || iy >= ny) continue;
-            cq[hy][hx] = load_cell<FROM_H>(P, s, m8, CI(ix, iy));
+    for (int st = B.id * (kTailThreads / 32) + (threadIdx.x >> 5); st < strips; st += warps) {
+        const int ix = (st % nsx) * kTailCols - 1 + lane, y0 = (st / nsx) * th, y1 = min(y0 + th, ny);
+        const bool own = lane >= 1 && lane <= kTailCols && ix < nx;
+        const bool xown = own || (lane >= 1 && ix == nx);   // writes its west face (ix = nx: the domain's east edge)
+        const bool xint = ix > 0 && ix < nx;
+        // Lanes beyond the grid read the nearest cell and face, rows beyond it the last row: every load
+        // is in bounds without a test, and what those lanes compute is not written.
+        const unsigned kx = min(max(ix, 0), nx - 1), kf = min(max(ix, 0), nx);
+        unsigned c = (unsigned)y0 * nx + kx, fx = (unsigned)y0 * (nx + 1) + kf;  // row iy's cell, west face; south face c
+        auto cell = [&](unsigned k) { return load_cell<FROM_H>(s, m8, k); };
+        auto yface = [&](unsigned k) { return FaceRaw{s.valid_y[k], s.b_y[k], s.ub_y[k]}; };
+        auto xface = [&](unsigned k) { return FaceRaw{s.valid_x[k], s.b_x[k], s.ub_x[k]}; };
+        auto put_y = [&](unsigned fi, bool interior, const FaceOut &o) {
+            if (interior && FROM_H) {
+                s.dhdy[fi] = o.dh;
+                s.dpwdy[fi] = o.dpw;
+            }
+            s.q_y[fi] = o.q;
+            s.Re_y[fi] = o.re;
+            if (L.kind != SHK_SLIDING_PRESCRIBED) s.taub_y[fi] = o.taub;
+        };
+        // the strip's first row and the faces below it
+        const CellRaw below = cell(y0 > 0 ? c - nx : c), first = cell(c);
+        const FaceRaw fs = yface(c);
+        CellRaw next_r = cell(y0 + 1 < ny ? c + nx : c);
+        FaceRaw north_r = yface(c + nx), west_r = xface(fx);
+        CellQ cur = make_cell<FROM_H>(P, first);
+        FaceSums S;
+        {
+            const CellQ q = make_cell<FROM_H>(P, below);
+            const FaceOut o = face<FROM_H, 1>(P, L, s, c, y0 > 0, q, cur, cur, fs);
+            if (own) put_y(c, y0 > 0, o);
+            S = face_sums(o);
         }
-        __syncthreads();
-        // (2) faces
-        for (int k = tid; k < kTailXF + kTailYF; k += kTailThreads) {
-            if (k < kTailXF) {
-                const int fc = k % (kTailW + 1), row = k / (kTailW + 1), f = x0 + fc, iy = y0 + row;
-                if (iy >= ny || f > nx) continue;
-                const bool interior = f > 0 && f < nx;
-                const CellQ &a = cq[row + 1][f > 0 ? fc : fc + 1];      // west cell (east cell at f = 0)
-                const CellQ &b = cq[row + 1][f < nx ? fc + 1 : fc];     // east cell (west cell at f = nx)
-                const size_t fi = XI(f, iy);
-                const FaceOut o = face<FROM_H>(P, L, s, 0, fi, interior, a, b, f > 0 ? a : b);
-                if ((fc < kTailW && f < nx) || f == nx) {
-                    if (interior && FROM_H) {
-                        s.dhdx[fi] = o.dh;
-                        s.dpwdx[fi] = o.dpw;
-                    }
-                    s.q_x[fi] = o.q;
-                    s.Re_x[fi] = o.re;
-                    if (L.kind != SHK_SLIDING_PRESCRIBED) s.taub_x[fi] = o.taub;
+        for (int iy = y0; iy < y1; iy++, c += nx, fx += nx + 1) {
+            const double G = s.G[c], bb = s.b[c], hp = CHECK ? h_prev[c] : 0.0;
+            // the next row's inputs
+            const bool more = iy + 1 < y1;
+            const unsigned cn = more ? c + nx : c;
+            const CellRaw next2_r = cell(iy + 2 < ny ? cn + nx : cn);
+            const FaceRaw north2_r = yface(cn + nx), west2_r = xface(more ? fx + nx + 1 : fx);
+            const CellQ nxt = make_cell<FROM_H>(P, next_r);
+            // north face
+            const bool nint = iy + 1 < ny;
+            const FaceOut on = face<FROM_H, 1>(P, L, s, c + nx, nint, cur, nxt, cur, north_r);
+            if (own && (more || !nint)) put_y(c + nx, nint, on);
+            const FaceSums Nf = face_sums(on);
+            // west face
+            CellQ w;
+            w.h = __shfl_up_sync(0xffffffffu, cur.h, 1);
+            w.pw = __shfl_up_sync(0xffffffffu, cur.pw, 1);
+            w.N = __shfl_up_sync(0xffffffffu, cur.N, 1);
+            w.lam = __shfl_up_sync(0xffffffffu, cur.lam, 1);
+            w.aub = __shfl_up_sync(0xffffffffu, cur.aub, 1);
+            const FaceOut ow = face<FROM_H, 0>(P, L, s, fx, xint, w, cur, ix > 0 ? w : cur, west_r);
+            if (xown) {
+                if (xint && FROM_H) {
+                    s.dhdx[fx] = ow.dh;
+                    s.dpwdx[fx] = ow.dpw;
                 }
-                fx[k] = FaceSm{o.re, o.ub * o.taub, o.q * o.dh, o.q * o.dpw};
-            } else {
-                const int kk = k - kTailXF, col = kk % kTailW, frow = kk / kTailW, ix = x0 + col, f = y0 + frow;
-                if (ix >= nx || f > ny) continue;
-                const bool interior = f > 0 && f < ny;
-                const CellQ &a = cq[f > 0 ? frow : frow + 1][col + 1];  // south cell (north cell at f = 0)
-                const CellQ &b = cq[f < ny ? frow + 1 : frow][col + 1]; // north cell (south cell at f = ny)
-                const size_t fi = YI(ix, f);
-                const FaceOut o = face<FROM_H>(P, L, s, 1, fi, interior, a, b, f > 0 ? a : b);
-                if ((frow < kTailH && f < ny) || f == ny) {
-                    if (interior && FROM_H) {
-                        s.dhdy[fi] = o.dh;
-                        s.dpwdy[fi] = o.dpw;
-                    }
-                    s.q_y[fi] = o.q;
-                    s.Re_y[fi] = o.re;
-                    if (L.kind != SHK_SLIDING_PRESCRIBED) s.taub_y[fi] = o.taub;
+                s.q_x[fx] = ow.q;
+                s.Re_x[fx] = ow.re;
+                if (L.kind != SHK_SLIDING_PRESCRIBED) s.taub_x[fx] = ow.taub;
+            }
+            const FaceSums W = face_sums(ow);
+            FaceSums E;
+            E.re = __shfl_down_sync(0xffffffffu, W.re, 1);
+            E.ut = __shfl_down_sync(0xffffffffu, W.ut, 1);
+            E.qd = __shfl_down_sync(0xffffffffu, W.qd, 1);
+            E.qp = __shfl_down_sync(0xffffffffu, W.qp, 1);
+            if (own) {
+                if (FROM_H) {
+                    s.pw[c] = cur.pw;
+                    s.N[c] = cur.N;
                 }
-                fy[kk] = FaceSm{o.re, o.ub * o.taub, o.q * o.dh, o.q * o.dpw};
+                // compute_Re! (src/water_flux.jl:107-112)
+                const double Re_c = (W.re + E.re + S.re + Nf.re) / 4;
+                s.Re[c] = Re_c;
+                // compute_mdot! (src/melt_rate.jl:106-137)
+                const double sh = fabs((E.ut + W.ut) / 2 + (Nf.ut + S.ut) / 2);
+                const double pot = fabs((E.qd + W.qd) / 2 + (Nf.qd + S.qd) / 2);
+                s.shear[c] = sh;
+                s.potential[c] = pot;
+                if (P.with_sensible) {
+                    const double sens = (E.qp + W.qp) / 2 + (Nf.qp + S.qp) / 2;
+                    s.sensible[c] = sens;
+                    s.mdot[c] = P.Linv * (G + sh + P.rho_w * P.g * pot + P.ct * P.cw * P.rho_w * sens);
+                } else {
+                    s.mdot[c] = P.Linv * (G + sh + P.rho_w * P.g * pot);
+                }
+                // compute_K! (src/water_flux.jl:221-226)
+                s.K[c] = (bb * bb * bb * P.g) / (12 * P.nu * (1 + P.omega * Re_c));
+                if (CHECK) {
+                    red[0] = jl_max(red[0], fabs(cur.h - hp));
+                    red[1] = jl_max(red[1], fabs(cur.h));
+                }
             }
+            S = Nf;
+            cur = nxt;
+            next_r = next2_r;
+            north_r = north2_r;
+            west_r = west2_r;
         }
-        __syncthreads();
-        // (3) cells
-        const int ix = x0 + tx, iy = y0 + ty;
-        if (tid < kTailW * kTailH && ix < nx && iy < ny) {
-            const size_t c = CI(ix, iy);
-            const CellQ &q0 = cq[ty + 1][tx + 1];
-            const FaceSm &W = fx[ty * (kTailW + 1) + tx], &E = fx[ty * (kTailW + 1) + tx + 1];
-            const FaceSm &S = fy[ty * kTailW + tx], &Nf = fy[(ty + 1) * kTailW + tx];
-            if (FROM_H) {
-                s.pw[c] = q0.pw;
-                s.N[c] = q0.N;
-            }
-            // compute_Re! (src/water_flux.jl:107-112)
-            const double Re_c = (W.re + E.re + S.re + Nf.re) / 4;
-            s.Re[c] = Re_c;
-            // compute_mdot! (src/melt_rate.jl:106-137)
-            const double sh = fabs((E.ut + W.ut) / 2 + (Nf.ut + S.ut) / 2);
-            const double pot = fabs((E.qd + W.qd) / 2 + (Nf.qd + S.qd) / 2);
-            s.shear[c] = sh;
-            s.potential[c] = pot;
-            if (P.with_sensible) {
-                const double sens = (E.qp + W.qp) / 2 + (Nf.qp + S.qp) / 2;
-                s.sensible[c] = sens;
-                s.mdot[c] = P.Linv * (s.G[c] + sh + P.rho_w * P.g * pot + P.ct * P.cw * P.rho_w * sens);
-            } else {
-                s.mdot[c] = P.Linv * (s.G[c] + sh + P.rho_w * P.g * pot);
-            }
-            // compute_K! (src/water_flux.jl:221-226)
-            const double bb = s.b[c];
-            s.K[c] = (bb * bb * bb * P.g) / (12 * P.nu * (1 + P.omega * Re_c));
-            if (CHECK) {
-                red[0] = jl_max(red[0], fabs(q0.h - h_prev[c]));
-                red[1] = jl_max(red[1], fabs(q0.h));
-            }
-        }
-        __syncthreads();  // the next tile reuses the shared arrays
     }
     if (CHECK) {
         double out[2];
@@ -557,11 +593,13 @@ int build_mask8(Ctx *c) {
     return check_launch(c, "k_mask8");
 }
 
-// One resident wave of the tail (kTailBlocksPerSm blocks per SM), striding over the tiles.
-static int tail_grid(const Ctx *c) {
-    const long long tiles = (long long)((c->nx + kTailW - 1) / kTailW) * ((c->ny + kTailH - 1) / kTailH);
-    return (int)std::max(1LL, std::min(tiles, (long long)c->num_sms * kTailBlocksPerSm));
+// One resident wave of the tail (kTailBlocksPerSm blocks per SM), or strips of two rows where those are fewer.
+int tail_blocks(int nx, int ny, int num_sms) {
+    const long long strips = (long long)((nx + kTailCols - 1) / kTailCols) * ((ny + 1) / 2);
+    const long long blocks = (strips + kTailThreads / 32 - 1) / (kTailThreads / 32);
+    return (int)std::max(1LL, std::min(blocks, (long long)num_sms * kTailBlocksPerSm));
 }
+static int tail_grid(const Ctx *c) { return tail_blocks(c->nx, c->ny, c->num_sms); }
 
 int launch_initial_conditions(Ctx *c) {
     const int nx = c->nx, ny = c->ny, n = nx * ny;

@@ -33,10 +33,8 @@ constexpr int kTX = 32;             // tile width (cells along x, one warp)
 constexpr int kTY = 8;              // tile height
 constexpr int kThreads = kTX * kTY; // 256 threads per block
 constexpr int kMaxRedValues = 4;
-// Resident blocks per SM of the fused field tail (288 threads).  Five (40 registers, a few spills)
-// measured fastest at 4096^2: 1310 us per call against 1376 with four, 1485 with six and 1616 with
-// three (no spills): the tail needs warps in flight more than registers.
-constexpr int kTailBlocksPerSm = 5;
+// The fused field tail: threads per block and resident blocks per SM (its registers: 128 a thread).
+constexpr int kTailThreads = 128, kTailBlocksPerSm = 4;
 // Resident blocks per SM of the assembly kernel (256 threads).  With every input loaded before the
 // cell's first branch (64 registers), four measured fastest at 4096^2: 406 us per call against
 // 419 with five (which spills); with the loads inside the branches, five had been fastest at
@@ -115,6 +113,8 @@ struct Params {
     int root3;           // n == 3: x^(1/n) as cbrt(x) (within an ulp of pow(x, 1/3.0))
     double Linv;         // 1/L
     double dx, dy, dx2, dy2;
+    double dx_inv, dy_inv;         // RN(1/dx), RN(1/dy): quotients by the grid spacing
+    double nu2x12, nu2x12_inv;     // 12 nu^2 and RN(1 / (12 nu^2))
 };
 
 struct Sliding {
@@ -247,6 +247,7 @@ int check_cuda(Ctx *c, cudaError_t e, const char *what);
 int check_launch(Ctx *c, const char *what);
 
 // shk_fields.cu
+int tail_blocks(int nx, int ny, int num_sms);
 int build_mask8(Ctx *c);
 int mg_set_first_wait_polls();
 int launch_initial_conditions(Ctx *c);

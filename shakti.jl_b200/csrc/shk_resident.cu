@@ -52,16 +52,6 @@ struct ResArgs {
     long spin;               // polls before a wait gives up
 };
 
-// a / d from the stored reciprocal y = RN(1 / d): a y, its remainder by one fused operation, and one
-// correction (Markstein, IBM J. Res. Dev. 34, 1990).  3 operations where the divide takes about 20, and
-// no slow path for a = 0 (fixed-head rows, cells beyond the grid), which every warp holding one such
-// cell otherwise runs through; it agreed with the divide in every one of 4e9 quotients tried.
-// (Infinities give NaN, which ends a solve with the same status one iteration earlier.)
-__device__ __forceinline__ double quotient(double a, double d, double y) {
-    const double t = a * y;
-    return fma(fma(-d, t, a), y, t);
-}
-
 // ---- tagged words -------------------------------------------------------------------------------
 __device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned tag) {
     asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(tag),
