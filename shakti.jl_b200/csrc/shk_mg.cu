@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "shk_device.cuh"
+#include "shk_mg_bottom.cuh"
 
 namespace shk {
 
@@ -1307,29 +1308,15 @@ __global__ void __launch_bounds__(128) k_mg_up_m(Lv L, const TB *b, const float 
 // operator in shared memory, cells mapped to 1024 threads and a block barrier after every phase, the
 // levels up to 32 x 32 took 24 us (0.7 us a phase), 20 % to 35 % of a multigrid iteration up to
 // 1024^2.  k_mg_bottom (nu = 2) keeps each thread's operator entries, right-hand side and iterate in
-// registers -- columns of 8, 2 and 1 cells on the three finest levels, 512 threads -- so that a phase
+// registers -- 8, 2 and 1 cells per thread on the three finest levels, 512 threads -- so that a phase
 // is a few shared-memory loads of neighbours and one barrier; the levels of at most 64 cells run in one
 // warp without block barriers.  That leaves room for the 64 x 64 level too, whose two tile kernels
-// took another 5 us each.  mg_bottom_body is the general form (any nu).
+// took another 5 us each.  From 64 x 64 down a launch is 19000 cycles (10 us), 2400 of them the one-warp
+// levels'; repeated in place it is 13000, the rest is instructions fetched for the first time.
+// mg_bottom_body is the general form (any nu).
 // ---------------------------------------------------------------------------------------------
 constexpr size_t kBottomBytesPerCell = 7 * sizeof(float) + 1;
 constexpr size_t kBottomBytes = 200 * 1024;
-constexpr int kBotThreads = 512;  // k_mg_bottom
-constexpr int kBotWarpCells = 64, kBotWarpLevels = 8;
-
-struct BottomLevel {
-    int nx, ny, off;  // offset of this level's cells in the shared arrays
-};
-struct BottomPlan {
-    int nlev, total;
-    BottomLevel lv[kMgMaxLevels];
-    const float *aE[kMgMaxLevels], *aN[kMgMaxLevels], *dP[kMgMaxLevels], *wD[kMgMaxLevels];
-    const uint8_t *act[kMgMaxLevels];
-    const int *done;
-    float s2;  // Lv::s2
-    int strips;  // levels above the one-warp ones (k_mg_bottom: columns of 8, 2 and 1 cells, coarsest last)
-};
-
 // Every loop over a level runs on a 2D thread map (32 columns x blockDim/32 rows), so no cell's
 // coordinates need an integer division; the arithmetic per cell is unchanged.
 __device__ __forceinline__ void mg_bottom_body(const BottomPlan &P, const float *b_top, float *x_top, int nu,
@@ -1436,279 +1423,19 @@ __global__ void __launch_bounds__(1024) k_mg_bottom_any(BottomPlan P, const floa
     mg_bottom_body(P, b_top, x_top, nu, wc);
 }
 
-// One level of k_mg_bottom: this thread's column of C cells.
-template <int C>
-struct BotStrip {
-    float E[C], W[C], N[C], D[C], w[C], b[C], x[C], S0;
-    unsigned act;
-    int nx, ny, ix, iy, c;  // the level's size; the strip's column, first row and first cell
-    bool on;
-
-    __device__ __forceinline__ bool in(int k) const { return on && iy + k < ny; }
-    __device__ __forceinline__ void load(const BottomPlan &P, int l) {
-        nx = P.lv[l].nx;
-        ny = P.lv[l].ny;
-        const int t = threadIdx.x, j = t / nx;
-        ix = t - j * nx;
-        iy = j * C;
-        on = iy < ny;
-        c = ix + iy * nx;
-        act = 0;
-        const float *aE = P.aE[l], *aN = P.aN[l], *dP = P.dP[l], *wD = P.wD[l];
-        const uint8_t *a = P.act[l];
-#pragma unroll
-        for (int k = 0; k < C; k++) {
-            const int q = c + k * nx;
-            const bool v = in(k);
-            E[k] = v ? aE[q] : 0.0f;
-            W[k] = v && ix > 0 ? aE[q - 1] : 0.0f;
-            N[k] = v ? aN[q] : 0.0f;
-            D[k] = v ? dP[q] : 0.0f;
-            w[k] = v ? wD[q] : 0.0f;
-            if (v && a[q]) act |= 1u << k;
-            x[k] = b[k] = 0.0f;
-        }
-        S0 = in(0) && iy > 0 ? aN[c - nx] : 0.0f;
-    }
-    __device__ __forceinline__ void put(float *X) const {
-#pragma unroll
-        for (int k = 0; k < C; k++)
-            if (in(k)) X[c + k * nx] = x[k];
-    }
-    // A x at the strip's cells; X holds every cell's x.
-    __device__ __forceinline__ void apply(const float *X, float (&y)[C]) const {
-        const float xs = on && iy > 0 ? X[c - nx] : 0.0f, xn = in(C) ? X[c + C * nx] : 0.0f;
-#pragma unroll
-        for (int k = 0; k < C; k++) {
-            const int q = c + k * nx;
-            const float xe = in(k) && ix < nx - 1 ? X[q + 1] : 0.0f, xw = in(k) && ix > 0 ? X[q - 1] : 0.0f;
-            const float xc = x[k];
-            float v = __fmul_rn(D[k], xc);
-            v = __fmaf_rn(E[k], __fsub_rn(xc, xe), v);
-            v = __fmaf_rn(W[k], __fsub_rn(xc, xw), v);
-            v = __fmaf_rn(N[k], __fsub_rn(xc, k < C - 1 ? x[k < C - 1 ? k + 1 : k] : xn), v);
-            v = __fmaf_rn(k > 0 ? N[k > 0 ? k - 1 : 0] : S0, __fsub_rn(xc, k > 0 ? x[k > 0 ? k - 1 : 0] : xs), v);
-            y[k] = v;
-        }
-    }
-    __device__ __forceinline__ void sweep(const float *X, float s) {
-        float y[C];
-        apply(X, y);
-#pragma unroll
-        for (int k = 0; k < C; k++) x[k] = __fmaf_rn(__fmul_rn(w[k], s), __fsub_rn(b[k], y[k]), x[k]);
-    }
-    // right-hand side from the finer level's residuals R
-    __device__ __forceinline__ void gather(const float *R, int nxf, int nyf) {
-#pragma unroll
-        for (int k = 0; k < C; k++) {
-            if (!in(k)) continue;
-            const int i = 2 * ix, j = 2 * (iy + k), f = i + j * nxf;
-            float v = 0.0f;
-            v += R[f];
-            if (i + 1 < nxf) v += R[f + 1];
-            if (j + 1 < nyf) {
-                v += R[f + nxf];
-                if (i + 1 < nxf) v += R[f + nxf + 1];
-            }
-            b[k] = v;
-        }
-    }
-    // descending half: two sweeps from zero, then the residual (0 on inactive cells) in X0
-    template <typename Sync>
-    __device__ __forceinline__ void down(float *X0, float *X1, float s2, Sync sync) {
-#pragma unroll
-        for (int k = 0; k < C; k++) x[k] = __fmul_rn(w[k], b[k]);
-        put(X0);
-        sync();
-        sweep(X0, s2);
-        put(X1);
-        sync();
-        float y[C];
-        apply(X1, y);
-#pragma unroll
-        for (int k = 0; k < C; k++)
-            if (in(k)) X0[c + k * nx] = act >> k & 1 ? __fsub_rn(b[k], y[k]) : 0.0f;
-        sync();
-    }
-    // ascending half: prolongation of the coarse result XC, two sweeps; the result in x
-    template <typename Sync>
-    __device__ __forceinline__ void up(float *X0, float *X1, const float *XC, int nxc, float wc, float s2, Sync sync) {
-#pragma unroll
-        for (int k = 0; k < C; k++)
-            if (act >> k & 1) x[k] = __fmaf_rn(wc, XC[(ix >> 1) + ((iy + k) >> 1) * nxc], x[k]);
-        put(X1);
-        sync();
-        sweep(X1, s2);
-        put(X0);
-        sync();
-        sweep(X0, 1.0f);
-    }
-};
-
-// The one-warp levels' operator, right-hand side and iterates.
-struct BotSmall {
-    float E[kBotWarpCells], N[kBotWarpCells], D[kBotWarpCells], w[kBotWarpCells], b[kBotWarpCells], X0[kBotWarpCells],
-        X1[kBotWarpCells];
-    uint8_t act[kBotWarpCells];
-};
-
-struct BotShared {
-    float X8[2][8 * kBotThreads], X2[2][2 * kBotThreads], X1[2][kBotThreads];
-    BotSmall sm[kBotWarpLevels];
-};
-
-// One cell of a one-warp level: A X at (ix, iy) = i.
-__device__ __forceinline__ float bot_ax(const BotSmall &S, const float *X, int nx, int ny, int ix, int iy, int i) {
-    const float xc = X[i];
-    float y = __fmul_rn(S.D[i], xc);
-    if (ix < nx - 1) y = __fmaf_rn(S.E[i], __fsub_rn(xc, X[i + 1]), y);
-    if (ix > 0) y = __fmaf_rn(S.E[i - 1], __fsub_rn(xc, X[i - 1]), y);
-    if (iy < ny - 1) y = __fmaf_rn(S.N[i], __fsub_rn(xc, X[i + nx]), y);
-    if (iy > 0) y = __fmaf_rn(S.N[i - nx], __fsub_rn(xc, X[i - nx]), y);
-    return y;
-}
-
-// The levels P.strips .. nlev - 1 by one warp; sm[0].b holds the right-hand side, the result ends in
-// sm[0].X1.
-__device__ __forceinline__ void bot_warp(const BottomPlan &P, BotSmall *sm, float wc, int lane) {
-    const int first = P.strips, n_lv = P.nlev - first;
-    auto each = [&](int l, auto f) {  // the lane's cells of level l
-        const int nx = P.lv[first + l].nx, ny = P.lv[first + l].ny;
-#pragma unroll
-        for (int t = 0; t < kBotWarpCells / 32; t++) {
-            const int i = lane + 32 * t;
-            if (i < nx * ny) f(i, i % nx, i / nx, nx, ny);
-        }
-        __syncwarp();
-    };
-    for (int l = 0; l < n_lv - 1; l++) {
-        BotSmall &S = sm[l], &G = sm[l + 1];
-        each(l, [&](int i, int, int, int, int) { S.X0[i] = __fmul_rn(S.w[i], S.b[i]); });
-        each(l, [&](int i, int ix, int iy, int nx, int ny) {
-            S.X1[i] = __fmaf_rn(__fmul_rn(S.w[i], P.s2), __fsub_rn(S.b[i], bot_ax(S, S.X0, nx, ny, ix, iy, i)), S.X0[i]);
-        });
-        each(l, [&](int i, int ix, int iy, int nx, int ny) {
-            S.X0[i] = S.act[i] ? __fsub_rn(S.b[i], bot_ax(S, S.X1, nx, ny, ix, iy, i)) : 0.0f;
-        });
-        const int nxf = P.lv[first + l].nx, nyf = P.lv[first + l].ny;
-        each(l + 1, [&](int i, int I, int J, int, int) {
-            const int f = 2 * I + 2 * J * nxf;
-            float v = 0.0f;
-            v += S.X0[f];
-            if (2 * I + 1 < nxf) v += S.X0[f + 1];
-            if (2 * J + 1 < nyf) {
-                v += S.X0[f + nxf];
-                if (2 * I + 1 < nxf) v += S.X0[f + nxf + 1];
-            }
-            G.b[i] = v;
-        });
-    }
-    {
-        BotSmall &S = sm[n_lv - 1];  // coarsest level: exact solve
-        each(n_lv - 1, [&](int i, int, int, int, int) { S.X1[i] = S.act[i] ? S.b[i] / S.D[i] : S.b[i]; });
-    }
-    for (int l = n_lv - 2; l >= 0; l--) {
-        BotSmall &S = sm[l], &G = sm[l + 1];
-        const int nxc = P.lv[first + l + 1].nx;
-        each(l, [&](int i, int ix, int iy, int, int) {
-            if (S.act[i]) S.X1[i] = __fmaf_rn(wc, G.X1[(ix >> 1) + (iy >> 1) * nxc], S.X1[i]);
-        });
-        each(l, [&](int i, int ix, int iy, int nx, int ny) {
-            S.X0[i] = __fmaf_rn(__fmul_rn(S.w[i], P.s2), __fsub_rn(S.b[i], bot_ax(S, S.X1, nx, ny, ix, iy, i)), S.X1[i]);
-        });
-        each(l, [&](int i, int ix, int iy, int nx, int ny) {
-            S.X1[i] = __fmaf_rn(S.w[i], __fsub_rn(S.b[i], bot_ax(S, S.X0, nx, ny, ix, iy, i)), S.X0[i]);
-        });
-    }
-}
-
-// nu = 2.  The levels are reached from the coarse end: strips = 0..3 levels above the one-warp ones.
 __device__ __forceinline__ void mg_bottom2_body(const BottomPlan &P, const float *b_top, float *x_top, float wc) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BotShared &M = *reinterpret_cast<BotShared *>(smem_raw);
-    const int tid = threadIdx.x, ns = P.strips, first = ns;
-    // every operator entry is requested before the stop flag is looked at
-    BotStrip<8> A8;
-    BotStrip<2> A2;
-    BotStrip<1> A1;
-    if (ns > 2) A8.load(P, ns - 3);
-    if (ns > 1) A2.load(P, ns - 2);
-    if (ns > 0) A1.load(P, ns - 1);
-    for (int l = first; l < P.nlev; l++) {
-        const int n = P.lv[l].nx * P.lv[l].ny;
-        BotSmall &S = M.sm[l - first];
-        const int i = tid & (kBotWarpCells - 1), part = tid / kBotWarpCells;
-        if (i < n) {
-            if (part == 0) S.E[i] = P.aE[l][i];
-            if (part == 1) S.N[i] = P.aN[l][i];
-            if (part == 2) S.D[i] = P.dP[l][i];
-            if (part == 3) S.w[i] = P.wD[l][i];
-            if (part == 4) S.act[i] = P.act[l][i];
-            if (part == 5 && ns == 0 && l == 0) S.b[i] = b_top[i];
-        }
-    }
-    auto top = [&](auto &A) {  // right-hand side of the finest level
+    BotOp O;
+    // every operator entry and the right-hand side are requested before the stop flag is looked at
+    bot_load(P, M, O);
+    bot_rhs(P, M, O, [&](const int (&i)[8], float (&v)[8], int n) {
 #pragma unroll
-        for (int k = 0; k < (int)(sizeof(A.b) / sizeof(float)); k++)
-            if (A.in(k)) A.b[k] = b_top[A.c + k * A.nx];
-    };
-    if (ns == 3) top(A8);
-    if (ns == 2) top(A2);
-    if (ns == 1) top(A1);
+        for (int k = 0; k < 8; k++)
+            if (k < n && i[k] >= 0) v[k] = b_top[i[k]];
+    });
     if (cg_finished(P.done)) return;  // (a block barrier)
-    auto block = [&]() { __syncthreads(); };
-    // the one-cell level: the warps that hold cells
-    const int n1 = ns > 0 ? A1.nx * A1.ny : 0, t1 = (n1 + 31) / 32 * 32;
-    auto some = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(t1) : "memory"); };
-    if (ns > 2) {
-        A8.down(M.X8[0], M.X8[1], P.s2, block);
-        A2.gather(M.X8[0], A8.nx, A8.ny);
-    }
-    if (ns > 1) {
-        A2.down(M.X2[0], M.X2[1], P.s2, block);
-        A1.gather(M.X2[0], A2.nx, A2.ny);
-    }
-    if (ns > 0 && tid < t1) A1.down(M.X1[0], M.X1[1], P.s2, some);
-    if (tid < 32) {
-        if (ns > 0) {
-            const int nx = P.lv[first].nx, ny = P.lv[first].ny, nxf = A1.nx, nyf = A1.ny;
-            for (int i = tid; i < nx * ny; i += 32) {
-                const int I = i % nx, J = i / nx, f = 2 * I + 2 * J * nxf;
-                float v = 0.0f;
-                v += M.X1[0][f];
-                if (2 * I + 1 < nxf) v += M.X1[0][f + 1];
-                if (2 * J + 1 < nyf) {
-                    v += M.X1[0][f + nxf];
-                    if (2 * I + 1 < nxf) v += M.X1[0][f + nxf + 1];
-                }
-                M.sm[0].b[i] = v;
-            }
-            __syncwarp();
-        }
-        bot_warp(P, M.sm, wc, tid);
-        if (ns == 0)
-            for (int i = tid; i < P.lv[0].nx * P.lv[0].ny; i += 32) x_top[i] = M.sm[0].X1[i];
-    }
-    if (ns == 0) return;
-    if (tid < t1) {
-        some();
-        A1.up(M.X1[0], M.X1[1], M.sm[0].X1, P.lv[first].nx, wc, P.s2, some);
-    }
-    if (ns == 1) {
-        if (A1.on) x_top[A1.c] = A1.x[0];
-        return;
-    }
-    if (tid < t1) A1.put(M.X1[1]);
-    __syncthreads();
-    A2.up(M.X2[0], M.X2[1], M.X1[1], A1.nx, wc, P.s2, block);
-    if (ns == 2) {
-        A2.put(x_top);
-        return;
-    }
-    A2.put(M.X2[1]);
-    __syncthreads();
-    A8.up(M.X8[0], M.X8[1], M.X2[1], A2.nx, wc, P.s2, block);
-    A8.put(x_top);
+    bot_run<1>(P, M, O, wc, [&](int i, float v) { x_top[i] = v; });
 }
 
 __global__ void __launch_bounds__(kBotThreads) k_mg_bottom(const __grid_constant__ BottomPlan P, const float *b_top,
@@ -2048,16 +1775,12 @@ static int fused_grid(const Ctx *c, const MgLevel &m) {
 }
 
 // The bottom kernel's levels, from the coarse end: those of at most 64 cells (one warp), then up to
-// three more whose columns of 1, 2 and 8 cells its threads hold.  Returns the finest (>= 1); *strips: how
+// three more of which a thread holds 1, 2 and 8 cells.  Returns the finest (>= 1); *strips: how
 // many of the three.
 static int bottom_level(const Ctx *c, int *strips = nullptr) {
     int lb = c->mg_levels - 1, ns = 0;
-    auto cells = [&](int l) { return (long long)c->mg[l].nx * c->mg[l].ny; };
-    while (lb > 1 && cells(lb - 1) <= kBotWarpCells && c->mg_levels - lb < kBotWarpLevels) lb--;
-    static const int column[3] = {1, 2, 8};
-    while (ns < 3 && lb > 1) {
-        const MgLevel &m = c->mg[lb - 1];
-        if ((long long)m.nx * ((m.ny + column[ns] - 1) / column[ns]) > kBotThreads) break;
+    while (lb > 1 && bot_fits(c->mg[lb - 1].nx, c->mg[lb - 1].ny, 0) && c->mg_levels - lb < kBotWarpLevels) lb--;
+    while (ns < 3 && lb > 1 && bot_fits(c->mg[lb - 1].nx, c->mg[lb - 1].ny, ns + 1)) {
         lb--;
         ns++;
     }

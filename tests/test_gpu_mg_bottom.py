@@ -24,7 +24,8 @@ def solve(shk, nx, ny, monkeypatch, bottom, law):
 # bottoms with 0, 1, 2 and 3 column levels above the one-warp levels; full and partly filled columns;
 # odd sizes on every level; long thin grids, whose levels shrink along one side only
 @pytest.mark.parametrize("nx,ny", [(2, 2), (5, 7), (16, 16), (17, 15), (31, 33), (64, 64), (65, 127), (128, 128),
-                                   (126, 130), (385, 301), (513, 250), (2, 700), (900, 3), (1040, 24), (520, 516)])
+                                   (126, 130), (385, 301), (513, 250), (2, 700), (900, 3), (1040, 24), (520, 516),
+                                   (8, 1500), (1026, 16), (4098, 5)])
 def test_bottom_kernel_matches_general_form(shk, cuda, monkeypatch, nx, ny):
     a, sa = solve(shk, nx, ny, monkeypatch, "1", shk.Arithmetic())
     b, sb = solve(shk, nx, ny, monkeypatch, "0", shk.Arithmetic())
