@@ -84,14 +84,22 @@ static int ctx_alloc(Ctx *c) {
         for (int k = 3; k < 9; k++) o_mg[l][k] = carve(m * sizeof(float)); // aE, aN, dP, wD, x0, x1
         o_mg[l][9] = carve(m * sizeof(float) + m);                       // b, then act bytes
     }
-    size_t vec_bytes = 0;
+    for (int l = 0; l < c->mg_levels; l++) {
+        c->mg[l].nx = dims[2 * l];
+        c->mg[l].ny = dims[2 * l + 1];
+    }
+    if (c->mg_resident) mg_res_plan(c);
+    size_t red_bytes = 0, halo_bytes = 0, vec_bytes = mg_res_vec_bytes(c);
     for (const ResPlan &P : c->res) {
         if (!P.blocks) continue;
-        c->res_red_bytes = std::max(c->res_red_bytes, res_red_bytes(P));
-        c->res_halo_bytes = std::max(c->res_halo_bytes, res_halo_bytes(P));
+        red_bytes = std::max(red_bytes, res_red_bytes(P));
+        halo_bytes = std::max(halo_bytes, res_halo_bytes(P));
         vec_bytes = std::max(vec_bytes, res_vec_bytes(P));
     }
-    const size_t o_red = carve(c->res_red_bytes), o_halo = carve(c->res_halo_bytes),
+    red_bytes = align_up(red_bytes, A);
+    halo_bytes = align_up(halo_bytes, A);
+    c->res_comm_bytes = red_bytes + halo_bytes + mg_res_comm_bytes(c);
+    const size_t o_comm = carve(c->res_comm_bytes),
                  // the scratch vectors take the place of the general kernels' Krylov vectors
                  o_vec = vec_bytes <= o_hprev - o_x ? o_x : carve(vec_bytes);
     size_t o_part = carve((size_t)kMaxRedValues * c->max_blocks * sizeof(double));
@@ -131,9 +139,11 @@ static int ctx_alloc(Ctx *c) {
         m.b = (float *)(b + o_mg[l][9]);
         m.act = (uint8_t *)(b + o_mg[l][9] + cnt * sizeof(float));
     }
-    c->res_red = (uint4 *)(b + o_red);
-    c->res_halo = (uint4 *)(b + o_halo);
-    c->res_vec = (double2 *)(b + o_vec);
+    c->res_comm = b + o_comm;
+    c->res_red = (uint4 *)(b + o_comm);
+    c->res_halo = (uint4 *)(b + o_comm + red_bytes);
+    c->mg_res_comm = b + o_comm + red_bytes + halo_bytes;
+    c->res_vec = c->mg_res_vec = (double2 *)(b + o_vec);
     c->partials = (double *)(b + o_part);
     c->counter = (unsigned int *)(b + o_cnt);
     c->dev = (DevScalars *)(b + o_dev);
@@ -295,6 +305,13 @@ SHK_API int shk_create(int nx, int ny, double lx, double ly, void *stream, void 
     const char *resident = getenv("SHK_CG_RESIDENT");
     if (resident ? atoi(resident) != 0 : c->mg_tma)
         for (int k = 0; k < 2; k++) c->res[k] = res_plan(nx, ny, c->num_sms, k == 1);
+    // SHK_MG_RESIDENT=0/1: the multigrid solves of small grids by the general kernels, or in one kernel
+    // (default, unless a switch asks for some of the general kernels)
+    c->mg_resident = true;
+    for (const char *name : {"SHK_MG_TMA", "SHK_MG_FUSED", "SHK_MG_CLUSTER", "SHK_MG_PAIR_X", "SHK_MG_BOTTOM", "SHK_MG_NU",
+                             "SHK_CG_GRAPHS"})
+        if (getenv(name)) c->mg_resident = false;
+    if (const char *v = getenv("SHK_MG_RESIDENT")) c->mg_resident = atoi(v) != 0;
     if (const char *v = getenv("SHK_TEST_RESIDENT_POLLS")) c->res_spin = std::max(0L, atol(v));
     c->max_blocks = c->grid_stencil > c->march_blocks ? c->grid_stencil : c->march_blocks;
     if (c->max_blocks < c->num_sms * 8) c->max_blocks = c->num_sms * 8;

@@ -163,13 +163,18 @@ struct Ctx {
     float mg_s2 = 1.0f;
     int mg_fused = 1;        // nu = 2 level kernels: 1 tile (default), 2 warp-marching, 0 per-sweep
     int mg_tma = 1;          // tile kernels stage through TMA copies where the level's pitch allows
+    bool mg_resident = true;  // the resident multigrid solve where the grid fits
     bool mg_bottom2 = true;   // the bottom levels by k_mg_bottom (else the general one-block form)
     bool mg_cluster = false;  // the coarse levels on one thread-block cluster (measured slower; opt-in)
     bool mg_pair_x = true;    // the outer CG's x updated once per two iterations (bit-identical x)
     struct MgTma *mg_maps = nullptr;  // the levels' tensor maps (built on first use)
     struct CgTma *cg_maps = nullptr;  // the plain Jacobi CG's tensor maps (built before its first capture)
     ResPlan res[2];           // the resident solve's geometry, Jacobi and Chebyshev (blocks = 0: does not fit)
-    size_t res_red_bytes = 0, res_halo_bytes = 0;
+    ResPlan mg_res;           // the resident multigrid solve's geometry
+    void *res_comm = nullptr; // every exchange buffer of the resident solves
+    size_t res_comm_bytes = 0;
+    void *mg_res_comm = nullptr;
+    double2 *mg_res_vec = nullptr;
     uint4 *res_red = nullptr, *res_halo = nullptr;  // its exchange buffers
     double2 *res_vec = nullptr;                     // its scratch vectors
     bool res_restart = false; // its tags start over at the next solve
@@ -278,6 +283,14 @@ size_t res_halo_bytes(const ResPlan &P);
 size_t res_vec_bytes(const ResPlan &P);
 bool res_serves(const Ctx *c, const shk_cg_opts *o);
 int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0);
+int res_tags(Ctx *c);
+
+// shk_mg_resident.cu
+void mg_res_plan(Ctx *c);
+size_t mg_res_comm_bytes(const Ctx *c);
+size_t mg_res_vec_bytes(const Ctx *c);
+bool mg_res_serves(const Ctx *c, const shk_cg_opts *o);
+int mg_res_solve(Ctx *c, const CgDev &init, const double *x0);
 
 // ensemble kernels: shk_fields.cu
 void ens_assemble(cudaStream_t s, EnsInst *E, const int *b2i, int nblocks);
@@ -316,6 +329,8 @@ enum { ENS_VC_INIT = 0, ENS_VC_ITER = 1 };
 // shk_mg.cu
 int mg_levels_for(int nx, int ny, int *dims, int maxl);
 int mg_setup(Ctx *c);
+int mg_bottom_start(const Ctx *c, int *strips);              // the bottom levels' finest
+int mg_bottom_plan(const Ctx *c, struct BottomPlan *P);      // fills P, returns the same
 void mg_release(Ctx *c);
 int mg_apply(Ctx *c, const double *r, double *z, CgDev *cg, bool init);
 bool mg_fuses_cg_update(const Ctx *c);

@@ -1080,7 +1080,7 @@ int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
     const CgDev &g = c->host_dev->cg;
     if (g.fault) {
         c->res_restart = true;
-        return fail(c, SHK_CUDA_ERROR, res_serves(c, o)
+        return fail(c, SHK_CUDA_ERROR, res_serves(c, o) || mg_res_serves(c, o)
                                            ? "an exchange of the resident solve did not complete (bounded wait ran out)"
                                            : "a TMA tile copy did not complete (bounded wait ran out)");
     }
@@ -1126,8 +1126,10 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
             return fail(c, SHK_BAD_ARG, "chebyshev nsteps must be in [2, 64]");
     }
     // the whole solve in one persistent kernel where the grid's Krylov state fits on the chip
-    if (res_serves(c, o)) {
-        int rc = res_solve(c, o, make_cg_init(o, n, false, 0.0), ws ? ws : c->st.h);
+    if (res_serves(c, o) || mg_res_serves(c, o)) {
+        const CgDev init = make_cg_init(o, n, false, 0.0);
+        const double *x0 = ws ? ws : c->st.h;
+        int rc = mg_res_serves(c, o) ? mg_res_solve(c, init, x0) : res_solve(c, o, init, x0);
         if (rc) return rc;
         if (deferred) {
             *deferred = true;

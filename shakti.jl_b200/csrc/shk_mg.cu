@@ -1806,6 +1806,14 @@ static size_t bottom_plan(const Ctx *c, int lb, BottomPlan *P) {
     return bottom2(c) ? sizeof(BotShared) : (size_t)off * kBottomBytesPerCell;
 }
 
+int mg_bottom_start(const Ctx *c, int *strips) { return bottom_level(c, strips); }
+int mg_bottom_plan(const Ctx *c, BottomPlan *P) {
+    const int lb = bottom_level(c);
+    bottom_plan(c, lb, P);
+    P->done = nullptr;
+    return lb;
+}
+
 // The cluster kernel's levels: lc = the finest level >= 1 whose slabs fit kClusterBytes, the CTA-0
 // levels from the first one with at most kCta0Cells cells.  False when the hierarchy has no level
 // to distribute (small grids: the one-block bottom kernel serves them).

@@ -1,0 +1,308 @@
+// shk_resident.cuh -- what the resident solves (shk_resident.cu, shk_mg_resident.cu) share: blocks that
+// own strips of whole rows, tagged words exchanged through L2, sums over every block, the operator on a
+// thread's two columns, and the CG scalars.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <float.h>
+
+#include "shk_device.cuh"
+
+namespace shk {
+
+constexpr int kResThreads = 512, kResWarps = kResThreads / 32;
+
+// The strips' geometry and the exchange buffers.
+struct ResComm {
+    int nx, ny, txp, ty;     // threads per row group (a multiple of 32), row groups per block
+    int groups;              // blocks that own strips
+    uint4 *red;              // [2][groups][4] tagged partials
+    uint4 *halo;             // [2][groups][2][2 * txp] tagged strip-edge rows
+    long spin;               // polls before a wait gives up
+};
+
+// ---- tagged words -------------------------------------------------------------------------------
+__device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned tag) {
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(tag),
+                 "r"(__double2hiint(v)), "r"(tag)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool ll_try(const uint4 *p, unsigned tag, double &v) {
+    unsigned lo, t0, hi, t1;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(lo), "=r"(t0), "=r"(hi), "=r"(t1)
+                 : "l"(p)
+                 : "memory");
+    v = __hiloint2double((int)hi, (int)lo);
+    return t0 == tag && t1 == tag;
+}
+
+// The scalars of the iteration, computed by one thread after a sum and published by a barrier: 16 warps
+// dividing for themselves keep the Float64 units busy longer than the barrier takes (us per iteration
+// every thread / one thread: 128^2 with R = 2 5.6 / 3.9, 512^2 with R = 2 6.9 / 5.5).
+struct CgScalars {
+    double alpha, beta, gamma, pnorm2, rz, rr;
+    long long iter;
+    int done, status;
+};
+struct ResSums {
+    double wred[3][kResWarps];   // a block's warp partials
+    double wsum[3][kResWarps];   // every block's partials, summed per polling warp
+    CgDev cg;
+    CgScalars sc;
+    int abort;
+};
+
+// After p'Ap: alpha, or zero curvature (k_cg_A's test).
+__device__ __forceinline__ void scalars_alpha(CgScalars &s, double pAp, double eps_curv) {
+    const double lim = eps_curv * s.pnorm2;
+    if ((pAp <= lim && fabs(pAp) <= lim) || isnan(pAp)) {
+        s.done = 1;
+        s.status = SHK_BREAKDOWN;
+    }
+    s.alpha = s.gamma / pAp;
+}
+// After r'z, r'r: beta (one thread), and the stopping test (another); cg_iter_finish's formulas.
+__device__ __forceinline__ void scalars_beta(CgScalars &s, double rz) {
+    const double beta = rz / s.gamma;
+    s.pnorm2 = rz + beta * beta * s.pnorm2;
+    s.gamma = rz;
+    s.beta = beta;
+}
+__device__ __forceinline__ void scalars_stop(CgScalars &s, const CgDev &cg, double rz, double rr) {
+    const bool krylov = cg.stop_rule == SHK_STOP_KRYLOV;
+    const double root = sqrt(krylov ? rz : rr);
+    const bool solved = root <= (krylov ? cg.eps_stop : cg.rtol * cg.bnorm) || (krylov && root + 1.0 <= 1.0);
+    s.rz = rz;
+    s.rr = rr;
+    s.iter += 1;
+    if (isnan(rz) || isnan(rr)) {
+        s.done = 1;
+        s.status = SHK_BREAKDOWN;
+    } else if (solved) {
+        s.done = 1;
+        s.status = SHK_OK;
+    } else if (s.iter >= cg.itmax) {
+        s.done = 1;
+        s.status = SHK_NOT_CONVERGED;
+    }
+}
+// The start (cg_init_finish) and the record of the solve.
+__device__ __forceinline__ void scalars_start(CgScalars &s, CgDev &cg, double rz, double rr, double bb) {
+    cg_init_finish(&cg, rz, rr, bb);
+    s.gamma = s.pnorm2 = s.rz = rz;
+    s.rr = rr;
+    s.alpha = s.beta = 0.0;
+    s.iter = 0;
+    s.done = cg.done;
+    s.status = cg.status;
+}
+__device__ __forceinline__ CgDev scalars_record(const CgScalars &s, CgDev g) {
+    g.done = 1;
+    g.status = s.status;
+    if (s.iter > 0) {
+        g.iter = s.iter;
+        g.rz_last = s.rz;
+        g.rr = sqrt(s.rr);
+        g.rnorm = g.stop_rule == SHK_STOP_KRYLOV ? sqrt(s.rz) : g.rr;
+        g.gamma = s.gamma;
+        g.beta = s.beta;
+        g.pNorm2 = s.pnorm2;
+        g.first = 0;
+    }
+    return g;
+}
+template <int R>
+struct Strip {
+    int tid, lane, warp, tx, gy, c0, row0;
+    bool act;                // owns columns
+    bool south, north;       // reads (and publishes) a strip-edge row across the block boundary
+    const double *op;        // aP, aE, aN: [array][row][column of the pair][kResThreads]
+    double *edge;            // [2 buffers][2 sides][R][kResWarps]
+    double *rows;            // [2 buffers][4][kResThreads]: first row (2 planes), last row (2 planes)
+    double aS0, aS1;         // the couplings below the first row
+};
+
+// The values a thread's columns exchange inside the block before the operator is applied: the outer
+// columns of each warp and the first and last row of each row group.
+template <int R>
+__device__ __forceinline__ void publish_block(const Strip<R> &S, const double (&v)[R][2], int buf, int ty) {
+    double *eL = S.edge + buf * 2 * R * kResWarps, *eR = eL + R * kResWarps;
+    if (S.lane == 0) {
+#pragma unroll
+        for (int j = 0; j < R; j++) eL[j * kResWarps + S.warp] = v[j][0];
+    }
+    if (S.lane == 31) {
+#pragma unroll
+        for (int j = 0; j < R; j++) eR[j * kResWarps + S.warp] = v[j][1];
+    }
+    if (ty > 1) {
+        double *w = S.rows + buf * 4 * kResThreads + S.tid;
+        w[0] = v[0][0];
+        w[kResThreads] = v[0][1];
+        w[2 * kResThreads] = v[R - 1][0];
+        w[3 * kResThreads] = v[R - 1][1];
+    }
+}
+
+// Rows of the neighbouring row groups of the same block (after the barrier that follows
+// publish_block); rows across the block boundary are left as they are.
+template <int R>
+__device__ __forceinline__ void group_rows(const Strip<R> &S, int buf, int txp, int ty, double (&s)[2], double (&n)[2]) {
+    const double *w = S.rows + buf * 4 * kResThreads;
+    if (S.gy > 0) {
+        s[0] = w[2 * kResThreads + S.tid - txp];
+        s[1] = w[3 * kResThreads + S.tid - txp];
+    }
+    if (S.gy < ty - 1) {
+        n[0] = w[S.tid + txp];
+        n[1] = w[kResThreads + S.tid + txp];
+    }
+}
+
+// out(j, y0, y1) for every row: y = A v, subtraction order E, W, N, S (stencil_apply).  Couplings
+// across the grid's edge are zero and the values beyond it finite, so no term needs a bounds test.
+template <int R, typename Out>
+__device__ __forceinline__ void apply_op(const Strip<R> &S, const double (&v)[R][2], const double (&vs)[2],
+                                         const double (&vn)[2], int buf, Out out) {
+    const double *eL = S.edge + buf * 2 * R * kResWarps, *eR = eL + R * kResWarps;
+    double s0 = vs[0], s1 = vs[1], a0 = S.aS0, a1 = S.aS1;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const double c0 = v[j][0], c1 = v[j][1];
+        double w = __shfl_up_sync(0xffffffffu, c1, 1), e = __shfl_down_sync(0xffffffffu, c0, 1);
+        if (S.lane == 0) w = S.warp > 0 ? eR[j * kResWarps + S.warp - 1] : 0.0;
+        if (S.lane == 31) e = S.warp < kResWarps - 1 ? eL[j * kResWarps + S.warp + 1] : 0.0;
+        constexpr int T = kResThreads;
+        const double *oP = S.op + 2 * j * T + S.tid, *oE = oP + 2 * R * T, *oN = oE + 2 * R * T;
+        const double E0 = oE[0], E1 = oE[T], N0 = oN[0], N1 = oN[T];
+        const double W0 = S.tx > 0 ? oE[T - 1] : 0.0;
+        const double n0 = j < R - 1 ? v[j < R - 1 ? j + 1 : j][0] : vn[0];
+        const double n1 = j < R - 1 ? v[j < R - 1 ? j + 1 : j][1] : vn[1];
+        double y0 = oP[0] * c0;
+        y0 -= E0 * c1;
+        y0 -= W0 * w;
+        y0 -= N0 * n0;
+        y0 -= a0 * s0;
+        double y1 = oP[T] * c1;
+        y1 -= E1 * e;
+        y1 -= E0 * c0;
+        y1 -= N1 * n1;
+        y1 -= a1 * s1;
+        out(j, y0, y1);
+        s0 = c0;
+        s1 = c1;
+        a0 = N0;
+        a1 = N1;
+    }
+}
+
+// Strip-edge rows across block boundaries: publish this block's first and last row, read the
+// neighbours' (the same threads do both, so a buffer two events old has been read).
+template <int R>
+__device__ __forceinline__ void send_rows(const ResComm &A, const Strip<R> &S, const double (&v)[R][2], int buf,
+                                          unsigned tag) {
+    uint4 *mine = A.halo + (((size_t)buf * A.groups + blockIdx.x) * 2) * (2 * A.txp) + S.c0;
+    if (S.south) {
+        ll_store(mine, v[0][0], tag);
+        ll_store(mine + 1, v[0][1], tag);
+    }
+    if (S.north) {
+        ll_store(mine + 2 * A.txp, v[R - 1][0], tag);
+        ll_store(mine + 2 * A.txp + 1, v[R - 1][1], tag);
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void recv_rows(const ResComm &A, const Strip<R> &S, int buf, unsigned tag, double (&s)[2],
+                                          double (&n)[2], volatile int *abort) {
+    const size_t per = 2 * (size_t)(2 * A.txp);
+    const uint4 *base = A.halo + (size_t)buf * A.groups * per + S.c0;
+    const long blk = blockIdx.x;
+    const uint4 *ps = base + (blk - 1) * (long)per + 2 * A.txp, *pn = base + (blk + 1) * (long)per;
+    bool s0 = !S.south, s1 = s0, n0 = !S.north, n1 = n0;
+    for (long i = 0; !(s0 && s1 && n0 && n1); i++) {
+        if (!s0) s0 = ll_try(ps, tag, s[0]);
+        if (!s1) s1 = ll_try(ps + 1, tag, s[1]);
+        if (!n0) n0 = ll_try(pn, tag, n[0]);
+        if (!n1) n1 = ll_try(pn + 1, tag, n[1]);
+        if (i >= A.spin || *abort) {
+            if (!(s0 && s1 && n0 && n1)) *abort = 1;
+            break;
+        }
+    }
+}
+
+// The total of a block's (or the polling warps') 16 values, the same bits in every lane.
+__device__ __forceinline__ double sum16(const double *w, int lane) {
+    double t = w[lane & 15];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// Sums v over every block: block partials, one tagged store per value; `meanwhile` (work that needs
+// no total); then every warp polls its share of the blocks' partials, at most one per lane, and the
+// warps' sums are added in the same order in every block.  One thread runs fin(totals), another
+// fin2(totals), and a barrier publishes what they leave.  Returns false when a wait ran out.
+template <int NV, typename Mid, typename Fin, typename Fin2>
+__device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane, int warp, double (&v)[NV], int buf,
+                                        unsigned tag, Mid meanwhile, Fin fin, Fin2 fin2) {
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        v[k] = warp_reduce<false>(v[k]);
+        if (lane == 0) sh.wred[k][warp] = v[k];
+    }
+    __syncthreads();
+    const int G = A.groups;  // (a block beyond them takes part in the totals without adding to them)
+    const bool alone = gridDim.x == 1;
+    uint4 *slots = A.red + (size_t)buf * G * 4;
+    double t[NV];
+    if (warp < 2) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) t[k] = sum16(sh.wred[k], lane);
+        if (warp == 0 && !alone && (int)blockIdx.x < G) {
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if (lane == k) ll_store(slots + blockIdx.x * 4 + k, t[k], tag);
+        }
+    }
+    meanwhile();
+    if (!alone) {
+        const int per = (G + kResWarps - 1) / kResWarps, i = warp * per + lane;  // per <= 16
+        double x[NV];
+#pragma unroll
+        for (int k = 0; k < NV; k++) x[k] = 0.0;
+        if (lane < per && i < G) {
+            for (long n = 0;; n++) {
+                bool ok = true;
+#pragma unroll
+                for (int k = 0; k < NV; k++) ok = ll_try(slots + i * 4 + k, tag, x[k]) && ok;
+                if (ok) break;
+                if (n >= A.spin || *(volatile int *)&sh.abort) {
+                    *(volatile int *)&sh.abort = 1;
+                    break;
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) x[k] += __shfl_down_sync(0xffffffffu, x[k], o);
+            if (lane == 0) sh.wsum[k][warp] = x[k];
+        }
+        __syncthreads();
+        if (warp < 2) {
+#pragma unroll
+            for (int k = 0; k < NV; k++) t[k] = sum16(sh.wsum[k], lane);
+        }
+    }
+    if (warp == 0 && lane == 0) fin(t);
+    if (warp == 1 && lane == 0) fin2(t);
+    __syncthreads();
+    return !*(volatile int *)&sh.abort;
+}
+
+} // namespace shk
