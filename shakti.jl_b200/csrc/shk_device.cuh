@@ -295,4 +295,37 @@ static __device__ void cg_iter_finish(CgDev *cg, double rz, double rr) {
     }
 }
 
+// Programmatic dependent launch.  The kernels of an iteration are a chain of launches of a few us each; a
+// kernel launched by launch_after starts while the previous one of its stream still runs, as soon as all of
+// that one's blocks run, and waits here until it has completed and its writes are visible.  Every block of
+// such a kernel calls after_previous before it reads what an earlier kernel of the chain wrote, before it
+// writes anything and before it leaves (so the chain's order is kept from end to end); only data that no
+// kernel of the chain writes may be read earlier.  (What the chain writes is not read through const
+// __restrict__ pointers in such a kernel: those loads may be moved up.)  `early` = false: an ordinary launch.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    next_may_start();
+}
+
+template <typename T>
+struct Same {
+    using type = T;
+};
+template <typename... P>
+static inline cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                       typename Same<P>::type... a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = early;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a...);
+}
+
 } // namespace shk

@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(kMarchX, 6) k_cg_A(int nx, int ny, int TH, con
                                                   T *__restrict__ Ap, CgDev *cg, double *partials,
                                                   unsigned int *counter, double eps_curv,
                                                   const T *__restrict__ dP = nullptr) {
+    next_may_start();
     cg_A_body<T, JAC, LAPL>(grid_blk(), nx, ny, TH, aP, aE, aN, r, zbuf, p_old, p_new, Ap, cg, partials, counter,
                             eps_curv, dP);
 }

@@ -522,6 +522,7 @@ __device__ __forceinline__ void mg_down_body(Blk B, const Lv &L, const TB *b, fl
 template <typename TB, bool FB = false>
 __global__ void __launch_bounds__(256, 6) k_mg_down(Lv L, const TB *b, float *xo, int nxc, int nyc, float *bc,
                                                     FusedB fbv = FusedB{}, const CgDev *cg = nullptr) {
+    after_previous();
     mg_down_body<TB, FB>(grid_blk(), L, b, xo, nxc, nyc, bc, fbv, cg);
 }
 
@@ -575,6 +576,7 @@ template <typename TB, bool LAST>
 __global__ void __launch_bounds__(256, 6) k_mg_up(Lv L, const TB *b, const float *xi, const float *xc, int nxc, float wc,
                                                   float *xo, double *z, CgDev *cg, int init, double *partials,
                                                   unsigned int *counter) {
+    after_previous();
     mg_up_body<TB, LAST>(grid_blk(), L, b, xi, xc, nxc, wc, xo, z, cg, init, partials, counter);
 }
 
@@ -821,6 +823,7 @@ __device__ __forceinline__ double2 rhs_pair(const float *SB, const Pair &P) {
 template <typename TB, bool FB>
 __global__ void __launch_bounds__(256, 3) k_mg_down_t(const __grid_constant__ TmaArgs M, Lv L, float *xo, int nxc,
                                                       int nyc, float *bc, FusedB fbv, CgDev *cg) {
+    after_previous();
     if constexpr (FB) {
         const CgView cv = block_cg_view(cg);
         if (cv.done) return;
@@ -915,6 +918,7 @@ template <typename TB, bool LAST>
 __global__ void __launch_bounds__(256, 4) k_mg_up_t(const __grid_constant__ TmaArgs M, Lv L, float wc, float *xo,
                                                     double *z, CgDev *cg, int init, double *partials,
                                                     unsigned int *counter) {
+    after_previous();
     if (cg_finished(L.done)) return;
     using Y = TLayout<TB, true, false>;
     extern __shared__ __align__(128) unsigned char sm[];
@@ -1012,6 +1016,7 @@ template <bool JAC>
 __global__ void __launch_bounds__(256, 4) k_cg_matvec_t(const __grid_constant__ MvArgs M, int nx, int ny,
                                                         double *p_new, double *Ap, CgDev *cg, double *partials,
                                                         unsigned int *counter, double eps_curv) {
+    after_previous();
     const CgView cv = block_cg_view(cg);
     if (cv.done) return;
     using Y = MvLayoutT<JAC>;
@@ -1427,8 +1432,9 @@ __device__ __forceinline__ void mg_bottom2_body(const BottomPlan &P, const float
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BotShared &M = *reinterpret_cast<BotShared *>(smem_raw);
     BotOp O;
-    // every operator entry and the right-hand side are requested before the stop flag is looked at
+    // the operator while the previous kernel runs; then the right-hand side, before the stop flag is looked at
     bot_load(P, M, O);
+    after_previous();
     bot_rhs(P, M, O, [&](const int (&i)[8], float (&v)[8], int n) {
 #pragma unroll
         for (int k = 0; k < 8; k++)
@@ -1764,6 +1770,12 @@ static float sweep_post(const Ctx *c, int s) { return s == 0 && c->mg_nu > 1 ? c
 // 959 us with the tile kernels, 1044 us with the marching ones).
 static bool fused(const Ctx *c) { return c->mg_fused && c->mg_nu == 2; }
 static bool marching(const Ctx *c) { return fused(c) && c->mg_fused == 2; }
+static long long tiles_of(const MgLevel &m) { return (long long)((m.nx + kFW - 1) / kFW) * ((m.ny + kFH - 1) / kFH); }
+// Which of an iteration's launches start while the previous one ends: those of one tile per block.  They are
+// launch latency (an iteration of 128 x 128 29.3 -> 25.8 us, 512 x 512 48.1 -> 44.9 us, a 1024 x 1024 step
+// 19.6 -> 18.9 ms, its level 0 launched the ordinary way).  Blocks that stride over several tiles lose by it:
+// with level 0 started early too, that step takes 19.2 ms and a 4096 x 4096 step 126.8 instead of 124.2 ms.
+static bool one_tile_each(const MgLevel &m, int grid) { return tiles_of(m) <= grid; }
 static int march_grid(const Ctx *c, const MgLevel &m) {
     const long long strips = (long long)((m.nx + kMW - 1) / kMW) * ((m.ny + kMH - 1) / kMH);
     return (int)std::max(1LL, std::min((strips + 3) / 4, (long long)c->max_blocks));
@@ -2144,7 +2156,7 @@ static int vcycle(Ctx *c, int l, CgDev *cg, int *res) {
         BottomPlan P;
         const size_t smem = bottom_plan(c, l, &P);
         P.done = done;
-        if (bottom2(c)) k_mg_bottom<<<1, kBotThreads, smem, c->stream>>>(P, m.b, m.x[0], wc);
+        if (bottom2(c)) launch_after(true, k_mg_bottom, 1, kBotThreads, smem, c->stream, P, m.b, m.x[0], wc);
         else k_mg_bottom_any<<<1, 1024, smem, c->stream>>>(P, m.b, m.x[0], c->mg_nu, wc);
         c->launches++;
         *res = 0;
@@ -2169,13 +2181,15 @@ static int vcycle(Ctx *c, int l, CgDev *cg, int *res) {
     if (trc) return trc;
     if (T && T->ok[l]) {
         const int gd = tma_grid(c, T, TK_DOWN, m), gu = tma_grid(c, T, TK_UP, m);
-        k_mg_down_t<float, false><<<gd, 256, TLayout<float, false, false>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gd), k_mg_down_t<float, false>, gd, 256, TLayout<float, false, false>::bytes,
+                     c->stream,
             tma_args(T, l, T->b[l], nullptr, nullptr), L, m.x[0], g.nx, g.ny, g.b, FusedB{}, cg);
         c->launches++;
         int gres = 0;
         int rc = vcycle(c, l + 1, cg, &gres);
         if (rc) return rc;
-        k_mg_up_t<float, false><<<gu, 256, TLayout<float, true, false>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gu), k_mg_up_t<float, false>, gu, 256, TLayout<float, true, false>::bytes,
+                     c->stream,
             tma_args(T, l, T->b[l], nullptr, &T->xc[l + 1][gres]), L, wc, m.x[1], nullptr, cg, 0, nullptr, nullptr);
         c->launches++;
         *res = 1;
@@ -2183,12 +2197,14 @@ static int vcycle(Ctx *c, int l, CgDev *cg, int *res) {
     }
     if (fused(c)) {
         const int gt = fused_grid(c, m);
-        k_mg_down<float><<<gt, 256, 0, c->stream>>>(L, m.b, m.x[0], g.nx, g.ny, g.b);
+        launch_after(one_tile_each(m, gt), k_mg_down<float>, gt, 256, 0, c->stream, L, m.b, m.x[0], g.nx, g.ny,
+                     g.b, FusedB{}, nullptr);
         c->launches++;
         int gres = 0;
         int rc = vcycle(c, l + 1, cg, &gres);
         if (rc) return rc;
-        k_mg_up<float, false><<<gt, 256, 0, c->stream>>>(L, m.b, m.x[0], g.x[gres], g.nx, wc, m.x[1], nullptr,
+        launch_after(one_tile_each(m, gt), k_mg_up<float, false>, gt, 256, 0, c->stream, L, m.b, m.x[0], g.x[gres],
+                     g.nx, wc, m.x[1], nullptr,
                                                          nullptr, 0, nullptr, nullptr);
         c->launches++;
         *res = 1;
@@ -2245,13 +2261,15 @@ int mg_apply(Ctx *c, const double *r, double *z, CgDev *cg, bool init) {
     if (trc) return trc;
     if (T && T->ok[0] && r_map(c, T, r)) {
         const int gd = tma_grid(c, T, TK_DOWN0, m), gu = tma_grid(c, T, TK_UP0, m);
-        k_mg_down_t<double, false><<<gd, 256, TLayout<double, false, false>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gd), k_mg_down_t<double, false>, gd, 256, TLayout<double, false,
+                     false>::bytes, c->stream,
             tma_args(T, 0, *r_map(c, T, r), nullptr, nullptr), L, m.x[0], g.nx, g.ny, g.b, FusedB{}, cg);
         c->launches++;
         int gres = 0;
         int rc = vcycle(c, 1, cg, &gres);
         if (rc) return rc;
-        k_mg_up_t<double, true><<<gu, 256, TLayout<double, true, false>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gu), k_mg_up_t<double, true>, gu, 256, TLayout<double, true, false>::bytes,
+                     c->stream,
             tma_args(T, 0, *r_map(c, T, r), nullptr, &T->xc[1][gres]), L, wc, nullptr, z, cg, init, c->partials,
             c->counter);
         c->launches++;
@@ -2259,12 +2277,14 @@ int mg_apply(Ctx *c, const double *r, double *z, CgDev *cg, bool init) {
     }
     if (fused(c)) {
         const int gt = fused_grid(c, m);
-        k_mg_down<double><<<gt, 256, 0, c->stream>>>(L, r, m.x[0], g.nx, g.ny, g.b);
+        launch_after(one_tile_each(m, gt), k_mg_down<double>, gt, 256, 0, c->stream, L, r, m.x[0], g.nx, g.ny, g.b,
+                     FusedB{}, nullptr);
         c->launches++;
         int gres = 0;
         int rc = vcycle(c, 1, cg, &gres);
         if (rc) return rc;
-        k_mg_up<double, true><<<gt, 256, 0, c->stream>>>(L, r, m.x[0], g.x[gres], g.nx, wc, nullptr, z, cg, init,
+        launch_after(one_tile_each(m, gt), k_mg_up<double, true>, gt, 256, 0, c->stream, L, r, m.x[0], g.x[gres],
+                     g.nx, wc, nullptr, z, cg, init,
                                                          c->partials, c->counter);
         c->launches++;
         return check_launch(c, "multigrid apply");
@@ -2307,7 +2327,8 @@ int mg_cg_matvec(Ctx *c, int par, const double *aP, const double *aE, const doub
         return SHK_OK;
     const MgLevel &m = c->mg[0];
     const MvArgs a{T->mv_z, T->mv_p[par], T->mv_aP, T->mv_aE, T->mv_aN};
-    k_cg_matvec_t<false><<<tma_grid(c, T, TK_MV, m), 256, MvLayout::bytes, c->stream>>>(
+    const int grid = tma_grid(c, T, TK_MV, m);
+    launch_after(one_tile_each(m, grid), k_cg_matvec_t<false>, grid, 256, MvLayout::bytes, c->stream,
         a, m.nx, m.ny, p_new, Ap, cg, c->partials, c->counter, eps_curv);
     *launched = true;
     return check_launch(c, "cg matvec");
@@ -2359,7 +2380,8 @@ int cg_jac_matvec(Ctx *c, int par, const double *r, const double *p_old, double 
     const long long tiles = (long long)((c->nx + kFW - 1) / kFW) * ((c->ny + kFH - 1) / kFH);
     const int grid = (int)std::max(1LL, std::min({tiles, (long long)c->max_blocks, (long long)T->grid}));
     const MvArgs a{T->r, T->p[par], T->aP, T->aE, T->aN};
-    k_cg_matvec_t<true><<<grid, 256, MvLayoutT<true>::bytes, c->stream>>>(a, c->nx, c->ny, p_new, Ap, cg,
+    launch_after(tiles <= grid, k_cg_matvec_t<true>, grid, 256, MvLayoutT<true>::bytes, c->stream, a, c->nx, c->ny,
+                 p_new, Ap, cg,
                                                                            c->partials, c->counter, eps_curv);
     *launched = true;
     return check_launch(c, "cg matvec (Jacobi)");
@@ -2382,14 +2404,16 @@ int mg_apply_fused_update(Ctx *c, const double *r_in, double *r_out, double *x, 
     if (trc) return trc;
     if (T && T->ok[0] && r_map(c, T, r_in) && r_map(c, T, r_out) && Ap == c->Ap) {
         const int gd = tma_grid(c, T, TK_DOWN0_FB, m), gu = tma_grid(c, T, TK_UP0, m);
-        k_mg_down_t<double, true><<<gd, 256, TLayout<double, false, true>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gd), k_mg_down_t<double, true>, gd, 256, TLayout<double, false, true>::bytes,
+                     c->stream,
             tma_args(T, 0, *r_map(c, T, r_in), &T->Ap, nullptr), L, m.x[0], g.nx, g.ny, g.b,
             FusedB{Ap, p, x, r_out, 0.0, p_prev, mode, pbuf, 0.0}, cg);
         c->launches++;
         int gres = 0;
         int rc = vcycle(c, 1, cg, &gres);
         if (rc) return rc;
-        k_mg_up_t<double, true><<<gu, 256, TLayout<double, true, false>::bytes, c->stream>>>(
+        launch_after(one_tile_each(m, gu), k_mg_up_t<double, true>, gu, 256, TLayout<double, true, false>::bytes,
+                     c->stream,
             tma_args(T, 0, *r_map(c, T, r_out), nullptr, &T->xc[1][gres]), L, wc, nullptr, z, cg, 0, c->partials,
             c->counter);
         c->launches++;
@@ -2397,13 +2421,15 @@ int mg_apply_fused_update(Ctx *c, const double *r_in, double *r_out, double *x, 
     }
     if (mode) return fail(c, SHK_CUDA_ERROR, "paired x updates need the TMA-staged level-0 kernel");
     const int gt = fused_grid(c, m);
-    k_mg_down<double, true><<<gt, 256, 0, c->stream>>>(L, r_in, m.x[0], g.nx, g.ny, g.b,
+    launch_after(one_tile_each(m, gt), k_mg_down<double, true>, gt, 256, 0, c->stream, L, r_in, m.x[0], g.nx, g.ny,
+                 g.b,
                                                         FusedB{Ap, p, x, r_out, 0.0}, cg);
     c->launches++;
     int gres = 0;
     int rc = vcycle(c, 1, cg, &gres);
     if (rc) return rc;
-    k_mg_up<double, true><<<gt, 256, 0, c->stream>>>(L, r_out, m.x[0], g.x[gres], g.nx, wc, nullptr, z, cg, 0,
+    launch_after(one_tile_each(m, gt), k_mg_up<double, true>, gt, 256, 0, c->stream, L, r_out, m.x[0], g.x[gres],
+                 g.nx, wc, nullptr, z, cg, 0,
                                                      c->partials, c->counter);
     c->launches++;
     return check_launch(c, "multigrid apply");
