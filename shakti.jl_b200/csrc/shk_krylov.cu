@@ -134,10 +134,11 @@ __device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
 // the diagonal excess computed in Float64 and rounded once.  Storing edge conductances and the
 // excess (rather than aP and the couplings) keeps the rounded operator accurate entry by entry
 // for this nearly singular M-matrix, whatever its condition number.
-template <typename T, bool JAC, bool LAPL>
+// TZ: the type zbuf is kept in (Float32 for the V-cycle's z, which is a Float32 value).
+template <typename T, bool JAC, bool LAPL, typename TZ = T>
 __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T *__restrict__ aP,
                                           const T *__restrict__ aE, const T *__restrict__ aN,
-                                          const T *__restrict__ r, const T *__restrict__ zbuf,
+                                          const T *__restrict__ r, const TZ *__restrict__ zbuf,
                                           const T *__restrict__ p_old, T *__restrict__ p_new, T *__restrict__ Ap,
                                           CgDev *cg, double *partials, unsigned int *counter, double eps_curv,
                                           const T *__restrict__ dP) {
@@ -155,7 +156,12 @@ __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T
     const bool inx = ix < nx;
     const int y1 = min(y0 + TH, ny);
     const int kfirst = y0 - 1, klast = y1;            // input rows kfirst..klast (clipped below)
-    const T *src_r = JAC ? r : zbuf;
+    using TR = std::conditional_t<JAC, T, TZ>;
+    const TR *src_r;
+    if constexpr (JAC) src_r = r;
+    else src_r = zbuf;
+    // row `slot`'s r or z in the ring
+    auto in_row = [&](int slot) -> TR * { return reinterpret_cast<TR *>(ring[slot][IR]); };
     // issue the copies of input row q into its ring slot (empty group when out of range)
     auto issue = [&](int q) {
         if (q >= 0 && q < ny && q <= klast) {
@@ -163,7 +169,7 @@ __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T
             const size_t rowoff = (size_t)q * nx;
             if (inx) {
                 const size_t c = rowoff + ix;
-                cp_async_elem(&ring[slot][IR][tid + 1], src_r + c);
+                cp_async_elem(&in_row(slot)[tid + 1], src_r + c);
                 cp_async_elem(&ring[slot][IP][tid + 1], aP + c);
                 if (!first) cp_async_elem(&ring[slot][IO][tid + 1], p_old + c);
                 cp_async_elem(&ring[slot][IE][tid + 1], aE + c);
@@ -172,14 +178,14 @@ __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T
             }
             if (tid == 0 && x0 > 0) {
                 const size_t c = rowoff + x0 - 1;
-                cp_async_elem(&ring[slot][IR][0], src_r + c);
+                cp_async_elem(&in_row(slot)[0], src_r + c);
                 if (JAC) cp_async_elem(&ring[slot][IP][0], aP + c);
                 if (!first) cp_async_elem(&ring[slot][IO][0], p_old + c);
                 cp_async_elem(&ring[slot][IE][0], aE + c);
             }
             if (tid == kMarchX - 1 && x0 + kMarchX < nx) {
                 const size_t c = rowoff + x0 + kMarchX;
-                cp_async_elem(&ring[slot][IR][W - 1], src_r + c);
+                cp_async_elem(&in_row(slot)[W - 1], src_r + c);
                 if (JAC) cp_async_elem(&ring[slot][IP][W - 1], aP + c);
                 if (!first) cp_async_elem(&ring[slot][IO][W - 1], p_old + c);
             }
@@ -187,7 +193,7 @@ __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T
         __pipeline_commit();
     };
     auto pform = [&](int slot, int j) -> T {
-        T z = JAC ? ring[slot][IR][j] / ring[slot][IP][j] : ring[slot][IR][j];
+        T z = JAC ? (T)in_row(slot)[j] / ring[slot][IP][j] : (T)in_row(slot)[j];
         return first ? z : z + beta * ring[slot][IO][j];
     };
     for (int q = kfirst; q < kfirst + R - 2; q++) issue(q);
@@ -261,16 +267,16 @@ __device__ __forceinline__ void cg_A_body(Blk B, int nx, int ny, int TH, const T
     }
 }
 
-template <typename T, bool JAC, bool LAPL = false>
+template <typename T, bool JAC, bool LAPL = false, typename TZ = T>
 __global__ void __launch_bounds__(kMarchX, 6) k_cg_A(int nx, int ny, int TH, const T *__restrict__ aP,
                                                   const T *__restrict__ aE, const T *__restrict__ aN,
-                                                  const T *__restrict__ r, const T *__restrict__ zbuf,
+                                                  const T *__restrict__ r, const TZ *__restrict__ zbuf,
                                                   const T *__restrict__ p_old, T *__restrict__ p_new,
                                                   T *__restrict__ Ap, CgDev *cg, double *partials,
                                                   unsigned int *counter, double eps_curv,
                                                   const T *__restrict__ dP = nullptr) {
     next_may_start();
-    cg_A_body<T, JAC, LAPL>(grid_blk(), nx, ny, TH, aP, aE, aN, r, zbuf, p_old, p_new, Ap, cg, partials, counter,
+    cg_A_body<T, JAC, LAPL, TZ>(grid_blk(), nx, ny, TH, aP, aE, aN, r, zbuf, p_old, p_new, Ap, cg, partials, counter,
                             eps_curv, dP);
 }
 
@@ -887,7 +893,7 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
             }
         }
         if (jac && lapl) {
-            k_cg_A<T, true, true><<<c->march_blocks, kMarchX, 0, c->stream>>>(
+            k_cg_A<T, true, true, T><<<c->march_blocks, kMarchX, 0, c->stream>>>(
                 nx, ny, c->march_th, aP, aE, aN, r, nullptr, p_old, p_new, Ap, cgd, c->partials, c->counter, eps_curv,
                 lapl);
         } else if (jac) {
@@ -899,12 +905,16 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
                 }
             }
             if (!launched)
-                k_cg_A<T, true><<<c->march_blocks, kMarchX, 0, c->stream>>>(nx, ny, c->march_th, aP, aE, aN, r,
+                k_cg_A<T, true, false, T><<<c->march_blocks, kMarchX, 0, c->stream>>>(nx, ny, c->march_th, aP, aE, aN, r,
                                                                            nullptr, p_old, p_new, Ap, cgd,
                                                                            c->partials, c->counter, eps_curv);
         } else if (lapl) {
             k_cg_A<T, false, true><<<c->march_blocks, kMarchX, 0, c->stream>>>(
                 nx, ny, c->march_th, aP, aE, aN, r, z, p_old, p_new, Ap, cgd, c->partials, c->counter, eps_curv, lapl);
+        } else if (fuse_update) {  // the V-cycle's z (mg_apply)
+            k_cg_A<T, false, false, float><<<c->march_blocks, kMarchX, 0, c->stream>>>(
+                nx, ny, c->march_th, aP, aE, aN, r, reinterpret_cast<const float *>(z), p_old, p_new, Ap, cgd,
+                c->partials, c->counter, eps_curv);
         } else {
             k_cg_A<T, false><<<c->march_blocks, kMarchX, 0, c->stream>>>(nx, ny, c->march_th, aP, aE, aN, r, z, p_old,
                                                                         p_new, Ap, cgd, c->partials, c->counter,
@@ -1376,7 +1386,7 @@ __global__ void __launch_bounds__(kMarchX, 6) k_ens_cg_A_mg(EnsInst *E, const in
     if (!I.pic_active) return;
     const double *p_old = parity ? I.p1 : I.p0;
     double *p_new = parity ? I.p0 : I.p1;
-    cg_A_body<double, false, false>(B, I.nx, I.ny, I.march_th, I.aP, I.aE, I.aN, I.r, I.z, p_old, p_new, I.Ap,
+    cg_A_body<double, false, false, float>(B, I.nx, I.ny, I.march_th, I.aP, I.aE, I.aN, I.r, (const float *)I.z, p_old, p_new, I.Ap,
                                     I.cg, I.partials, I.counter, DBL_EPSILON, nullptr);
 }
 
@@ -1386,7 +1396,7 @@ __global__ void __launch_bounds__(kMarchX, 6) k_ens_cg_A(EnsInst *E, const int *
     if (!I.pic_active) return;
     const double *p_old = parity ? I.p1 : I.p0;
     double *p_new = parity ? I.p0 : I.p1;
-    cg_A_body<double, true, false>(B, I.nx, I.ny, I.march_th, I.aP, I.aE, I.aN, I.r, nullptr, p_old, p_new, I.Ap,
+    cg_A_body<double, true, false, double>(B, I.nx, I.ny, I.march_th, I.aP, I.aE, I.aN, I.r, nullptr, p_old, p_new, I.Ap,
                                    I.cg, I.partials, I.counter, DBL_EPSILON, nullptr);
 }
 
@@ -1545,7 +1555,7 @@ extern "C" SHK_API int shk_cg_solve_static(int nx, int ny, const double *aP, con
         }
         for (int k = 0; k < batch; k++, enq++) {
             double *p_old = p[enq & 1], *p_new = p[(enq + 1) & 1];
-            k_cg_A<double, true><<<march_blocks, kMarchX, 0, s>>>(nx, ny, march_th, aP, aE, aN, r, nullptr, p_old,
+            k_cg_A<double, true, false, double><<<march_blocks, kMarchX, 0, s>>>(nx, ny, march_th, aP, aE, aN, r, nullptr, p_old,
                                                                   p_new, Ap, cg, partials, counter, DBL_EPSILON);
             k_cg_B<double, true><<<grid_b, kThreads, 0, s>>>(n, aP, p_new, Ap, xc, r, cg, partials, counter);
         }

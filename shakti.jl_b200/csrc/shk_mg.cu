@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(256, 6) k_mg_down(Lv L, const TB *b, float *xo
 // otherwise it writes the level's result to xo.
 template <typename TB, bool LAST>
 __device__ __forceinline__ void mg_up_body(Blk B, const Lv &L, const TB *b, const float *xi, const float *xc, int nxc,
-                                           float wc, float *xo, double *z, CgDev *cg, int init, double *partials,
+                                           float wc, float *xo, float *z, CgDev *cg, int init, double *partials,
                                            unsigned int *counter) {
     if (cg_finished(L.done)) return;
     __shared__ FusedSm S;
@@ -553,9 +553,9 @@ __device__ __forceinline__ void mg_up_body(Blk B, const Lv &L, const TB *b, cons
             const size_t q = (size_t)gx + (size_t)gy * L.nx;
             if (LAST) {
                 const double rk = r64[hy * kFSW + hx];
-                const double zk = (double)__fmaf_rn(S.wD[hy][hx], __fsub_rn((float)rk, ax), S.x1[hy][hx]);
+                const float zk = __fmaf_rn(S.wD[hy][hx], __fsub_rn((float)rk, ax), S.x1[hy][hx]);
                 z[q] = zk;
-                red[0] += rk * zk;
+                red[0] += rk * (double)zk;
                 red[1] += rk * rk;
             } else {
                 xo[q] = __fmaf_rn(S.wD[hy][hx], __fsub_rn(S.b[hy][hx], ax), S.x1[hy][hx]);
@@ -574,7 +574,7 @@ __device__ __forceinline__ void mg_up_body(Blk B, const Lv &L, const TB *b, cons
 
 template <typename TB, bool LAST>
 __global__ void __launch_bounds__(256, 6) k_mg_up(Lv L, const TB *b, const float *xi, const float *xc, int nxc, float wc,
-                                                  float *xo, double *z, CgDev *cg, int init, double *partials,
+                                                  float *xo, float *z, CgDev *cg, int init, double *partials,
                                                   unsigned int *counter) {
     after_previous();
     mg_up_body<TB, LAST>(grid_blk(), L, b, xi, xc, nxc, wc, xo, z, cg, init, partials, counter);
@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(256, 3) k_mg_down_t(const __grid_constant__ Tm
 // k_mg_up on TMA-staged tiles.
 template <typename TB, bool LAST>
 __global__ void __launch_bounds__(256, 4) k_mg_up_t(const __grid_constant__ TmaArgs M, Lv L, float wc, float *xo,
-                                                    double *z, CgDev *cg, int init, double *partials,
+                                                    float *z, CgDev *cg, int init, double *partials,
                                                     unsigned int *counter) {
     after_previous();
     if (cg_finished(L.done)) return;
@@ -965,11 +965,11 @@ __global__ void __launch_bounds__(256, 4) k_mg_up_t(const __grid_constant__ TmaA
                 const size_t q = (size_t)gx + (size_t)gy * L.nx;
                 if (LAST) {
                     const double2 rk = rhs_pair<Y>(SB, P0);
-                    const double z0 = (double)__fmaf_rn(P0.W.x, __fsub_rn((float)rk.x, ax.x), x1.x);
-                    const double z1 = (double)__fmaf_rn(P0.W.y, __fsub_rn((float)rk.y, ax.y), x1.y);
-                    *reinterpret_cast<double2 *>(z + q) = make_double2(z0, z1);
-                    red[0] += rk.x * z0;
-                    red[0] += rk.y * z1;
+                    const float z0 = __fmaf_rn(P0.W.x, __fsub_rn((float)rk.x, ax.x), x1.x);
+                    const float z1 = __fmaf_rn(P0.W.y, __fsub_rn((float)rk.y, ax.y), x1.y);
+                    *reinterpret_cast<float2 *>(z + q) = make_float2(z0, z1);
+                    red[0] += rk.x * (double)z0;
+                    red[0] += rk.y * (double)z1;
                     red[1] += rk.x * rk.x;
                     red[1] += rk.y * rk.y;
                 } else {
@@ -990,9 +990,12 @@ __global__ void __launch_bounds__(256, 4) k_mg_up_t(const __grid_constant__ TmaA
 // p_new = z + beta p_old over the tile and a one-cell ring, then Ap = A p_new on the tile and
 // p_new'Ap, with the Float64 roundings of k_cg_A (no fused multiply-adds: every product and sum is
 // rounded, in k_cg_A's order, so the two kernels agree bit for bit up to the order of the grid
-// sum).  Boxes: z and p_old over rows y0-1 .. y0+16 and columns x0-2 .. x0+33 (36 x 18), aP on
+// sum).  z is the V-cycle's last sweep, a Float32 value, and is kept as one: 8 bytes a cell less of the 148 an
+// iteration moves on level 0.  Boxes: p_old over rows y0-1 .. y0+16 and columns x0-2 .. x0+33 (36 x 18), z two
+// columns more on each side, aP on
 // the tile, aE from column x0-2 (34 x 16), aN from row y0-1 (32 x 17).
 constexpr int kMvW = kFW + 4, kMvH = kFH + 2;  // staged p region (36 x 18)
+constexpr int kMvZW = kFW + 8;                 // staged z: Float32, two columns more on each side (16-byte boxes)
 
 struct MvArgs {
     CUtensorMap z, po, aP, aE, aN;
@@ -1004,9 +1007,9 @@ constexpr unsigned rnd128(unsigned v) { return (v + 127u) & ~127u; }
 // staged over the same 36 x 18 region as r and p_old.
 template <bool JAC = false>
 struct MvLayoutT {
-    static constexpr unsigned pB = kMvW * kMvH * 8, apB = JAC ? pB : kFW * kFH * 8, aeB = (kFW + 2) * kFH * 8,
+    static constexpr unsigned pB = kMvW * kMvH * 8, zB = JAC ? pB : kMvZW * kMvH * 4, apB = JAC ? pB : kFW * kFH * 8, aeB = (kFW + 2) * kFH * 8,
                               anB = kFW * (kFH + 1) * 8;
-    static constexpr unsigned o_z = 0, o_po = rnd128(pB), o_aP = rnd128(o_po + pB), o_aE = rnd128(o_aP + apB),
+    static constexpr unsigned o_z = 0, o_po = rnd128(zB), o_aP = rnd128(o_po + pB), o_aE = rnd128(o_aP + apB),
                               o_aN = rnd128(o_aE + aeB), stage = rnd128(o_aN + anB);
     static constexpr unsigned o_p = 2 * stage, o_bar = rnd128(o_p + pB), bytes = o_bar + 16;
 };
@@ -1025,7 +1028,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_matvec_t(const __grid_constant__ 
     const bool first = cv.first != 0;
     const double beta = cv.beta;
     const int tid = threadIdx.x;
-    const unsigned tx = Y::pB * (first ? 1 : 2) + Y::apB + Y::aeB + Y::anB;
+    const unsigned tx = Y::zB + (first ? 0 : Y::pB) + Y::apB + Y::aeB + Y::anB;
     // p pairs: slot 0 = pair tid of the 324, slot 1 = pair 256 + tid (tid < 68)
     constexpr int np = kMvW / 2, npairs = np * kMvH;
     const int k0 = (tid / np) * kMvW + 2 * (tid % np), k1 = ((tid + 256) / np) * kMvW + 2 * ((tid + 256) % np);
@@ -1036,7 +1039,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_matvec_t(const __grid_constant__ 
         nx, ny, sm, cg,
         [&](unsigned char *st, uint64_t *b, int x0, int y0) {
             tma_expect(b, tx);
-            tma_load(st + Y::o_z, &M.z, b, x0 - 2, y0 - 1);
+            tma_load(st + Y::o_z, &M.z, b, JAC ? x0 - 2 : x0 - 4, y0 - 1);
             if (!first) tma_load(st + Y::o_po, &M.po, b, x0 - 2, y0 - 1);
             if (JAC) tma_load(st + Y::o_aP, &M.aP, b, x0 - 2, y0 - 1);
             else tma_load(st + Y::o_aP, &M.aP, b, x0, y0);
@@ -1045,14 +1048,18 @@ __global__ void __launch_bounds__(256, 4) k_cg_matvec_t(const __grid_constant__ 
         },
         [&](int, int) {},
         [&](unsigned char *st, int x0, int y0) {
-            const double *Z = reinterpret_cast<const double *>(st + Y::o_z);
             const double *PO = reinterpret_cast<const double *>(st + Y::o_po);
             const double *APh = reinterpret_cast<const double *>(st + Y::o_aP);
             auto form = [&](int k) {
-                double2 z = *reinterpret_cast<const double2 *>(Z + k);  // JAC: r
+                double2 z;
                 if (JAC) {  // outside the grid r = aP = 0 gives NaN there, a value no output reads
+                    const double2 r = *reinterpret_cast<const double2 *>(reinterpret_cast<const double *>(st + Y::o_z) + k);
                     const double2 d = *reinterpret_cast<const double2 *>(APh + k);
-                    z = make_double2(__ddiv_rn(z.x, d.x), __ddiv_rn(z.y, d.y));
+                    z = make_double2(__ddiv_rn(r.x, d.x), __ddiv_rn(r.y, d.y));
+                } else {
+                    const float2 f = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(st + Y::o_z) + k +
+                                                                       (k / kMvW) * (kMvZW - kMvW) + 2);
+                    z = make_double2((double)f.x, (double)f.y);
                 }
                 double2 v = z;
                 if (!first) {
@@ -2066,7 +2073,7 @@ static MgTma *tma_maps(Ctx *c, int *rc) {
     }
     if (T->ok[0]) {
         const MgLevel &m = c->mg[0];
-        T->mv_ok = encode(fn, &T->mv_z, F64, 8, c->z, m.nx, m.ny, kMvW, kMvH) &&
+        T->mv_ok = encode(fn, &T->mv_z, F32, 4, c->z, m.nx, m.ny, kMvZW, kMvH) &&
                    encode(fn, &T->mv_p[0], F64, 8, c->p[0], m.nx, m.ny, kMvW, kMvH) &&
                    encode(fn, &T->mv_p[1], F64, 8, c->p[1], m.nx, m.ny, kMvW, kMvH) &&
                    encode(fn, &T->mv_aP, F64, 8, c->aP, m.nx, m.ny, kFW, kFH) &&
@@ -2270,7 +2277,7 @@ int mg_apply(Ctx *c, const double *r, double *z, CgDev *cg, bool init) {
         if (rc) return rc;
         launch_after(one_tile_each(m, gu), k_mg_up_t<double, true>, gu, 256, TLayout<double, true, false>::bytes,
                      c->stream,
-            tma_args(T, 0, *r_map(c, T, r), nullptr, &T->xc[1][gres]), L, wc, nullptr, z, cg, init, c->partials,
+            tma_args(T, 0, *r_map(c, T, r), nullptr, &T->xc[1][gres]), L, wc, nullptr, (float *)z, cg, init, c->partials,
             c->counter);
         c->launches++;
         return check_launch(c, "multigrid apply");
@@ -2284,7 +2291,7 @@ int mg_apply(Ctx *c, const double *r, double *z, CgDev *cg, bool init) {
         int rc = vcycle(c, 1, cg, &gres);
         if (rc) return rc;
         launch_after(one_tile_each(m, gt), k_mg_up<double, true>, gt, 256, 0, c->stream, L, r, m.x[0], g.x[gres],
-                     g.nx, wc, nullptr, z, cg, init,
+                     g.nx, wc, nullptr, (float *)z, cg, init,
                                                          c->partials, c->counter);
         c->launches++;
         return check_launch(c, "multigrid apply");
@@ -2414,7 +2421,7 @@ int mg_apply_fused_update(Ctx *c, const double *r_in, double *r_out, double *x, 
         if (rc) return rc;
         launch_after(one_tile_each(m, gu), k_mg_up_t<double, true>, gu, 256, TLayout<double, true, false>::bytes,
                      c->stream,
-            tma_args(T, 0, *r_map(c, T, r_out), nullptr, &T->xc[1][gres]), L, wc, nullptr, z, cg, 0, c->partials,
+            tma_args(T, 0, *r_map(c, T, r_out), nullptr, &T->xc[1][gres]), L, wc, nullptr, (float *)z, cg, 0, c->partials,
             c->counter);
         c->launches++;
         return check_launch(c, "multigrid apply");
@@ -2429,7 +2436,7 @@ int mg_apply_fused_update(Ctx *c, const double *r_in, double *r_out, double *x, 
     int rc = vcycle(c, 1, cg, &gres);
     if (rc) return rc;
     launch_after(one_tile_each(m, gt), k_mg_up<double, true>, gt, 256, 0, c->stream, L, r_out, m.x[0], g.x[gres],
-                 g.nx, wc, nullptr, z, cg, 0,
+                 g.nx, wc, nullptr, (float *)z, cg, 0,
                                                      c->partials, c->counter);
     c->launches++;
     return check_launch(c, "multigrid apply");
@@ -2581,7 +2588,7 @@ __global__ void __launch_bounds__(256, 6) k_ens_mg_up0(EnsInst *E, const EnsMg *
     const Lv L{m.nx, m.ny, m.aE, m.aN, m.dP, m.wD, m.act, &I.cg->done, G.s2};
     const double *r = init ? I.r : (parity ? I.r : I.r2);  // the iteration's new residual buffer
     const float *xc = g.x[1 == G.lb ? 0 : 1];
-    mg_up_body<double, true>(q.B, L, r, m.x[0], xc, g.nx, G.wc, nullptr, I.z, I.cg, init, I.partials, I.counter);
+    mg_up_body<double, true>(q.B, L, r, m.x[0], xc, g.nx, G.wc, nullptr, (float *)I.z, I.cg, init, I.partials, I.counter);
 }
 
 int ens_mg_plan(Ctx *c, EnsMgPlan *plan) {
