@@ -39,7 +39,8 @@ UNIT = "timesteps/s"
 # Algorithmic bytes per cell of one CG iteration.  Jacobi (Float64): k_cg_A reads aP, aE, aN, r,
 # p_old and writes p_new, Ap; k_cg_B reads aP, p_new, Ap, x, r and writes x, r (14 words).  With the
 # multigrid preconditioner, k_cg_A reads z instead of r (7 words) and the x/r update is counted
-# with the V-cycle's first kernel (mg_vcycle_bytes).
+# with the V-cycle's first kernel (mg_vcycle_bytes).  The counts are the algorithm's: the kernels keep
+# the multigrid form's z as a Float32 value and move 4 bytes less on each side of it.
 CG_BYTES = {"plain": 14 * 8, "fp32cg": 14 * 4, "multigrid": 7 * 8}
 FORMS = {"multigrid": "Float64 CG + Float32 aggregation-multigrid V-cycle preconditioner",
          "plain": "Float64 CG, Jacobi (the reference algorithm)",
