@@ -276,8 +276,8 @@ struct BotQuad {
 // A one-warp level: per cell the operator with all four couplings (zeros beyond the level), the right-hand
 // side, and the cell's place in this level's array, its first child's in the finer level's and its parent's
 // in the coarser's.  A level of at most 32 cells lies one cell to a lane and reads its neighbours by
-// shuffles (a phase of sub-warp levels takes about 100 cycles so; through shared memory, with the
-// coordinates' divisions in every phase, it took about 1500); its child is then the finer level's lane (bits 5 and 6: the second column, the second row
+// shuffles (about 110 cycles a phase; with every level in shared memory, bounds tests and the coordinates'
+// divisions in every phase the one-warp levels took 20000 cycles a V-cycle, now 2400); its child is then the finer level's lane (bits 5 and 6: the second column, the second row
 // exist), its parent the coarser level's lane, and X0 holds its iterate by lanes.
 struct BotSmall {
     float E[kBotWarpCells], W[kBotWarpCells], N[kBotWarpCells], S[kBotWarpCells], D[kBotWarpCells], w[kBotWarpCells],
