@@ -51,7 +51,8 @@ struct ResSums {
     double wsum[3][kResWarps];   // every block's partials, summed per polling warp
     CgDev cg;
     CgScalars sc;
-    int abort;
+    int abort;                   // a wait of this block ran out
+    int left;                    // abort as the last sum left it, the same for every thread
 };
 
 // After p'Ap: alpha, or zero curvature (k_cg_A's test).
@@ -245,7 +246,9 @@ __device__ __forceinline__ double sum16(const double *w, int lane) {
 // Sums v over every block: block partials, one tagged store per value; `meanwhile` (work that needs
 // no total); then every warp polls its share of the blocks' partials, at most one per lane, and the
 // warps' sums are added in the same order in every block.  One thread runs fin(totals), another
-// fin2(totals), and a barrier publishes what they leave.  Returns false when a wait ran out.
+// fin2(totals), and a barrier publishes what they leave.  Returns false when a wait ran out: to the
+// whole block, so the flag is taken between two barriers (a warp that has left the last one may
+// already be in its next wait and set it).
 template <int NV, typename Mid, typename Fin, typename Fin2>
 __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane, int warp, double (&v)[NV], int buf,
                                         unsigned tag, Mid meanwhile, Fin fin, Fin2 fin2) {
@@ -299,10 +302,13 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
             for (int k = 0; k < NV; k++) t[k] = sum16(sh.wsum[k], lane);
         }
     }
-    if (warp == 0 && lane == 0) fin(t);
+    if (warp == 0 && lane == 0) {
+        sh.left = *(volatile int *)&sh.abort;
+        fin(t);
+    }
     if (warp == 1 && lane == 0) fin2(t);
     __syncthreads();
-    return !*(volatile int *)&sh.abort;
+    return !*(volatile int *)&sh.left;
 }
 
 } // namespace shk

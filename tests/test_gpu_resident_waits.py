@@ -1,0 +1,62 @@
+"""The bounded waits of the resident solves (shk_resident.cuh), cut short."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HOOKS = ("POLLS",)
+
+
+class Problem:
+    """A perturbed state and its solver; `hooks` are the test switches a context reads when it is created."""
+
+    def __init__(self, shk, monkeypatch, nx, ny, precond, resident=True, **hooks):
+        for k in HOOKS:
+            monkeypatch.delenv("SHK_TEST_RESIDENT_" + k, raising=False)
+        for k, v in hooks.items():
+            monkeypatch.setenv("SHK_TEST_RESIDENT_" + k, str(v))
+        for k in ("CG", "MG"):
+            monkeypatch.setenv(f"SHK_{k}_RESIDENT", "1" if resident else "0")
+        import torch
+        w = shk.configs.plain(nx, 97.0 * (nx - 1), ny=ny, ly=101.0 * (ny - 1), C=0.25)
+        self.shk, self.g, self.p, self.sl = shk, shk.Grid(nx, ny, w.lx, w.ly), shk.ModelParameters(), \
+            shk.RegularizedCoulombSlidingLaw(0.25)
+        self.s = shk.State(self.g)
+        shk.set_initial_conditions(self.s, self.g, self.p, self.sl, **w.inputs)
+        gen = torch.Generator("cuda").manual_seed(5)
+        self.s.h += torch.randn((ny, nx), generator=gen, device="cuda", dtype=torch.float64).t()
+        self.h0 = self.s.h.clone()
+        self.kw = dict(chebyshev_degree=4 if precond == "chebyshev" else None, multigrid=precond == "multigrid")
+
+    def solver(self, **kw):
+        return self.shk.CGIterativeSolver(self.g, self.shk.MatrixFreeLinearSystem, stop_rule="relres", atol=0.0,
+                                          **self.kw, **kw)
+
+    def solve(self, **kw):
+        """(head, stats), or the error and None; from the same head every time."""
+        self.s.h.copy_(self.h0)
+        try:
+            st = self.shk.solve_elliptic_linear_system(self.solver(**kw), self.s, self.g, self.p,
+                                                       self.shk.Arithmetic(), self.sl)
+        except self.shk._lib.ShaktiError as e:
+            assert "did not complete" in str(e)
+            return e, None
+        return self.s.h.cpu().numpy(), st
+
+
+FORMS = [(201, 150, "jacobi"), (640, 300, "jacobi"), (64, 64, "chebyshev"), (513, 301, "chebyshev"),
+         (200, 150, "multigrid"), (385, 301, "multigrid")]
+
+
+@pytest.mark.parametrize("nx,ny,precond", FORMS)
+def test_a_block_whose_wait_ran_out_leaves_as_a_whole(shk, cuda, monkeypatch, nx, ny, precond):
+    """Whichever warps of a block see the wait run out first: every call returns, and a context with its
+    waits whole solves as before."""
+    kw = dict(rtol=0.0, itmax=6)
+    want, _ = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
+    for polls in (0, 1, 2, 3, 5, 8):
+        q = Problem(shk, monkeypatch, nx, ny, precond, POLLS=polls)
+        for _ in range(5):
+            q.solve(**kw)
+    h, _ = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
+    assert np.array_equal(h, want)
