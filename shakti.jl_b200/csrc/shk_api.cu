@@ -312,7 +312,10 @@ SHK_API int shk_create(int nx, int ny, double lx, double ly, void *stream, void 
                              "SHK_CG_GRAPHS"})
         if (getenv(name)) c->mg_resident = false;
     if (const char *v = getenv("SHK_MG_RESIDENT")) c->mg_resident = atoi(v) != 0;
-    if (const char *v = getenv("SHK_TEST_RESIDENT_POLLS")) c->res_spin = std::max(0L, atol(v));
+    // tests of the resident solves' waits (ResComm): their limit, in one block, from one iteration on
+    if (const char *v = getenv("SHK_TEST_RESIDENT_POLLS")) c->res_test_spin = std::max(0, atoi(v));
+    if (const char *v = getenv("SHK_TEST_RESIDENT_BLOCK")) c->res_test_block = atoi(v);
+    if (const char *v = getenv("SHK_TEST_RESIDENT_ITER")) c->res_test_iter = std::max(0, atoi(v));
     c->max_blocks = c->grid_stencil > c->march_blocks ? c->grid_stencil : c->march_blocks;
     if (c->max_blocks < c->num_sms * 8) c->max_blocks = c->num_sms * 8;
     rc = mg_set_first_wait_polls();

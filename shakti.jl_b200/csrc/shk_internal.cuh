@@ -178,7 +178,8 @@ struct Ctx {
     uint4 *res_red = nullptr, *res_halo = nullptr;  // its exchange buffers
     double2 *res_vec = nullptr;                     // its scratch vectors
     bool res_restart = false; // its tags start over at the next solve
-    long res_spin = 1L << 21; // polls before one of its waits gives up
+    int res_spin = 1 << 21;   // polls before one of its waits gives up
+    int res_test_spin = -1, res_test_block = -1, res_test_iter = 0; // tests: ResComm's (-1: none)
     int max_blocks = 0;
     int grid_stencil = 0;    // blocks for tile-stride kernels
     int march_th = 8;        // row-marching tile height
@@ -284,6 +285,7 @@ size_t res_vec_bytes(const ResPlan &P);
 bool res_serves(const Ctx *c, const shk_cg_opts *o);
 int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0);
 int res_tags(Ctx *c);
+void res_waits(const Ctx *c, struct ResComm &a);
 
 // shk_mg_resident.cu
 void mg_res_plan(Ctx *c);

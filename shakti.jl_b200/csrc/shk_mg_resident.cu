@@ -62,38 +62,28 @@ struct MgResArgs : ResComm {
 __device__ __forceinline__ void ll_store(uint2 *p, float v, unsigned tag) {
     asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
 }
-__device__ __forceinline__ float ll_wait(const uint2 *p, unsigned tag, long spin, volatile int *abort) {
+__device__ __forceinline__ float ll_wait(const uint2 *p, unsigned tag, volatile ResWait &W) {
     unsigned v = 0, t = 0;
-    for (long i = 0;; i++) {
+    for (int i = 0;; i++) {
         asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v), "=r"(t) : "l"(p) : "memory");
-        if (t == tag) break;
-        if (i >= spin || *abort) {
-            *abort = 1;
-            break;
-        }
+        if (t == tag || wait_over(W, i)) break;
     }
     return __uint_as_float(v);
 }
 
 // Two words, or two pairs of adjacent words (16-byte aligned), polled together; a null pointer is not read.
-__device__ __forceinline__ void ll_wait2(const uint2 *pa, const uint2 *pb, unsigned tag, float &a, float &b, long spin,
-                                         volatile int *abort) {
-    for (long k = 0;; k++) {
+__device__ __forceinline__ void ll_wait2(const uint2 *pa, const uint2 *pb, unsigned tag, float &a, float &b, volatile ResWait &W) {
+    for (int k = 0;; k++) {
         unsigned va = 0, ta = tag, vb = 0, tb = tag;
         if (pa) asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(va), "=r"(ta) : "l"(pa) : "memory");
         if (pb) asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(vb), "=r"(tb) : "l"(pb) : "memory");
         a = __uint_as_float(va);
         b = __uint_as_float(vb);
-        if (ta == tag && tb == tag) break;
-        if (k >= spin || *abort) {
-            *abort = 1;
-            break;
-        }
+        if ((ta == tag && tb == tag) || wait_over(W, k)) break;
     }
 }
-__device__ __forceinline__ void ll_wait2(const uint4 *pa, const uint4 *pb, unsigned tag, float2 &a, float2 &b, long spin,
-                                         volatile int *abort) {
-    for (long k = 0;; k++) {
+__device__ __forceinline__ void ll_wait2(const uint4 *pa, const uint4 *pb, unsigned tag, float2 &a, float2 &b, volatile ResWait &W) {
+    for (int k = 0;; k++) {
         uint4 x = make_uint4(0, tag, 0, tag), y = x;
         if (pa)
             asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -107,11 +97,7 @@ __device__ __forceinline__ void ll_wait2(const uint4 *pa, const uint4 *pb, unsig
                          : "memory");
         a = make_float2(__uint_as_float(x.x), __uint_as_float(x.z));
         b = make_float2(__uint_as_float(y.x), __uint_as_float(y.z));
-        if (x.y == tag && x.w == tag && y.y == tag && y.w == tag) break;
-        if (k >= spin || *abort) {
-            *abort = 1;
-            break;
-        }
+        if ((x.y == tag && x.w == tag && y.y == tag && y.w == tag) || wait_over(W, k)) break;
     }
 }
 __device__ __forceinline__ void ll_store(uint2 *p, float2 v, unsigned tag) {  // p 16-byte aligned
@@ -121,9 +107,8 @@ __device__ __forceinline__ void ll_store(uint2 *p, float2 v, unsigned tag) {  //
 }
 
 // n words at p[i[k]], all requested before any is looked at.
-__device__ __forceinline__ void ll_wait_all(const uint2 *p, const int (&i)[8], float (&v)[8], int n, unsigned tag, long spin,
-                                            volatile int *abort) {
-    for (long k = 0;; k++) {
+__device__ __forceinline__ void ll_wait_all(const uint2 *p, const int (&i)[8], float (&v)[8], int n, unsigned tag, volatile ResWait &W) {
+    for (int k = 0;; k++) {
         unsigned t[8];
         bool all = true;
 #pragma unroll
@@ -136,11 +121,7 @@ __device__ __forceinline__ void ll_wait_all(const uint2 *p, const int (&i)[8], f
         }
 #pragma unroll
         for (int m = 0; m < 8; m++) all = all && t[m] == tag;
-        if (all) break;
-        if (k >= spin || *abort) {
-            *abort = 1;
-            break;
-        }
+        if (all || wait_over(W, k)) break;
     }
 }
 
@@ -206,10 +187,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
     const unsigned tag0 = *A.epoch;  // every block reads it before the first sum; block 0 writes it after the last
     unsigned st = tag0, vt = tag0, ht = tag0;  // tags of sums, V-cycles and row exchanges
     int rb = 0;
-    volatile int *abort = &sh.abort;
+    volatile ResWait &W = sh.wait;
     if (tid == 0) {
         sh.cg = A.init;
-        sh.abort = 0;
+        wait_limit(A, W, 0);
     }
     auto nothing = [&]() {};
     CgScalars &sc = sh.sc;
@@ -225,9 +206,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         for (bool first = true;; first = false) {  // (one place for the V-cycle: its registers stay registers)
             vt++;
             bot_rhs(A.bp, M, O, [&](const int (&i)[8], float (&v)[8], int n) {
-                ll_wait_all(A.gather, i, v, n, vt, A.spin, abort);
+                ll_wait_all(A.gather, i, v, n, vt, W);
             });
             __syncthreads();
+            if (W.abort) {  // a result from part of a right-hand side is not handed on
+                ok = false;
+                break;
+            }
             bot_run<2>(A.bp, M, O, A.wc, [&](int i, float v) { ll_store(A.scatter + i, v, vt); });
             __syncthreads();
             rb ^= 1;
@@ -242,7 +227,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
             if (!ok || sc.done) break;
             rb ^= 1;
             ok = all_sum<1>(
-                A, sh, lane, warp, v1, rb, ++st, nothing, [&](double (&t)[1]) { scalars_alpha(sc, t[0], A.eps_curv); },
+                A, sh, lane, warp, v1, rb, ++st, nothing,
+                [&](double (&t)[1]) {
+                    scalars_alpha(sc, t[0], A.eps_curv);
+                    wait_limit(A, W, sc.iter + 1);
+                },
                 [](double (&)[1]) {});
             if (!ok || sc.done) break;
         }
@@ -332,7 +321,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         dt = ++ht;
         send_rows<R>(A, S, v, hb, dt);
     };
-    auto recv64 = [&](double (&s)[2], double (&n)[2]) { recv_rows<R>(A, S, hb, dt, s, n, abort); };
+    auto recv64 = [&](double (&s)[2], double (&n)[2]) { recv_rows<R>(A, S, hb, dt, s, n, W); };
     auto share = [&](const double (&v)[R][2], double (&s)[2], double (&n)[2]) {
         publish_block<R>(S, v, 0, ty);
         __syncthreads();
@@ -360,7 +349,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
             float2 a, b;
             ll_wait2(S.south ? reinterpret_cast<const uint4 *>(base + ((size_t)(blk - 1) * 2 + 1) * pitch) : nullptr,
                      S.north ? reinterpret_cast<const uint4 *>(base + (size_t)(blk + 1) * 2 * pitch) : nullptr, t, a, b,
-                     A.spin, abort);
+                     W);
             if (S.south) *reinterpret_cast<float2 *>(X + S.c0) = a;
             if (S.north) *reinterpret_cast<float2 *>(X + (size_t)(brows + 1) * pitch + S.c0) = b;
         }
@@ -404,7 +393,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         for (int x = tid; x < M.nx; x += T) {
             float a, b;
             ll_wait2(blk > 0 ? base + ((size_t)(blk - 1) * 2 + 1) * M.nx + x : nullptr,
-                     blk + 1 < G ? base + (size_t)(blk + 1) * 2 * M.nx + x : nullptr, t, a, b, A.spin, abort);
+                     blk + 1 < G ? base + (size_t)(blk + 1) * 2 * M.nx + x : nullptr, t, a, b, W);
             if (blk > 0) X[x] = a;
             if (blk + 1 < G) X[(M.rows + 1) * M.nx + x] = b;
         }
@@ -521,7 +510,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
                 float v = M.X1[M.nx + i];
                 const int k = (xx >> 1) + (y >> 1) * nxc;
                 const float c = more ? C.X0[C.nx + k]
-                                     : ll_wait(A.scatter + (size_t)(M.y0 >> 1) * nxc + k, vt, A.spin, abort);
+                                     : ll_wait(A.scatter + (size_t)(M.y0 >> 1) * nxc + k, vt, W);
                 if (M.act[i]) v = __fmaf_rn(A.wc, c, v);
                 M.X0[M.nx + i] = v;
                 edge(M, l, t, xx, y, v);
@@ -538,7 +527,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
                 const int yc = (S.gy * R + j) / 2;
                 float c;
                 if (A.nd > 1) c = MgSm(smem, A.lv[1]).X0[(1 + yc) * nxc + S.tx];
-                else c = ll_wait(A.scatter + (size_t)(blk * (brows / 2) + yc) * nxc + S.tx, vt, A.spin, abort);
+                else c = ll_wait(A.scatter + (size_t)(blk * (brows / 2) + yc) * nxc + S.tx, vt, W);
 #pragma unroll
                 for (int f = 0; f < 4; f++)
                     if (act >> (2 * j + f) & 1) x[j + (f >> 1)][f & 1] = __fmaf_rn(A.wc, c, x[j + (f >> 1)][f & 1]);
@@ -655,7 +644,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         rb ^= 1;
         ok = all_sum<1>(
             A, sh, lane, warp, v, rb, ++st, [&]() { recv64(as, an); },
-            [&](double (&t)[1]) { scalars_alpha(sc, t[0], A.eps_curv); }, [](double (&)[1]) {});
+            [&](double (&t)[1]) {
+                scalars_alpha(sc, t[0], A.eps_curv);
+                wait_limit(A, W, sc.iter + 1);
+            },
+            [](double (&)[1]) {});
         if (!ok || sc.done) break;
         alpha = sc.alpha;
 #pragma unroll
@@ -766,7 +759,7 @@ int mg_res_solve(Ctx *c, const CgDev &init, const double *x0) {
     a.txp = P.txp;
     a.ty = P.ty;
     a.groups = P.blocks;
-    a.spin = c->res_spin;
+    res_waits(c, a);
     a.nd = mg_bottom_plan(c, &a.bp);
     unsigned char *b = (unsigned char *)c->mg_res_comm;
     auto take = [&](size_t bytes) {

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     int hb = 0, rb = 0, sb = 0;  // halo, sum and shared-memory buffers in turn
     if (S.tid == 0) {
         sh.cg = A.init;
-        sh.abort = 0;
+        wait_limit(A, sh.wait, 0);
         if (CHEB) {
             ch.lam_min = A.cheb->lam_min;
             ch.lam_max = A.cheb->lam_max;
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
         send_rows<R>(A, S, v, hb, tag);
         s[0] = s[1] = n[0] = n[1] = 0.0;
         share(v, s, n);
-        recv_rows<R>(A, S, hb, tag, s, n, &sh.abort);
+        recv_rows<R>(A, S, hb, tag, s, n, sh.wait);
     };
     auto nothing = [&]() {};
     bool ok = true;
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     };
     double ps[2] = {0.0, 0.0}, pn[2] = {0.0, 0.0};  // p on the rows below and above the thread's
     double zs[2] = {0.0, 0.0}, zn[2] = {0.0, 0.0};  // z there
-    auto recv_z = [&]() { recv_rows<R>(A, S, hb, tag - 1, zs, zn, &sh.abort); };
+    auto recv_z = [&]() { recv_rows<R>(A, S, hb, tag - 1, zs, zn, sh.wait); };
 
     // ---- start: r = b - A x0, z, r'z, r'r, b'b (GROUNDED rows) ------------------------------------
     if (ok) {
@@ -401,7 +401,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
         rb ^= 1;
         ok = all_sum<1>(
             A, sh, S.lane, S.warp, v, rb, ++tag, nothing,
-            [&](double (&t)[1]) { scalars_alpha(sc, t[0], A.eps_curv); }, [](double (&)[1]) {});
+            [&](double (&t)[1]) {
+                scalars_alpha(sc, t[0], A.eps_curv);
+                wait_limit(A, sh.wait, sc.iter + 1);
+            },
+            [](double (&)[1]) {});
         if (!ok || sc.done) break;
         const double alpha = sc.alpha;
         double w[2] = {0.0, 0.0};
@@ -721,6 +725,13 @@ int res_tags(Ctx *c) {
     return check_cuda(c, e, "resident solve buffers");
 }
 
+void res_waits(const Ctx *c, ResComm &a) {
+    a.spin = c->res_spin;
+    a.test_spin = c->res_test_spin;
+    a.test_block = c->res_test_block;
+    a.test_iter = c->res_test_spin < 0 ? -1 : c->res_test_iter;
+}
+
 // One solve: h = x0 + the correction; the scalars end in c->dev->cg.  Asynchronous.
 int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0) {
     if (int rc = res_tags(c)) return rc;
@@ -758,7 +769,7 @@ int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0)
     a.halo = c->res_halo;
     a.epoch = &c->dev->res_epoch;
     a.eps_curv = DBL_EPSILON;
-    a.spin = c->res_spin;
+    res_waits(c, a);
     return cheb ? res_launch_rows<true>(c, a) : res_launch_rows<false>(c, a);
 }
 

@@ -18,8 +18,30 @@ struct ResComm {
     int groups;              // blocks that own strips
     uint4 *red;              // [2][groups][4] tagged partials
     uint4 *halo;             // [2][groups][2][2 * txp] tagged strip-edge rows
-    long spin;               // polls before a wait gives up
+    int spin;                // polls before a wait gives up
+    // tests: test_spin polls instead, in block test_block (-1: in every block) from the last sum of iteration
+    // test_iter on (0: from the start)
+    int test_spin, test_block, test_iter;
 };
+
+// A block's waits (in its shared memory): one that runs out makes the whole block leave.
+struct ResWait {
+    int abort;               // a wait of this block ran out
+    int spin;                // polls that a wait has
+};
+__device__ __forceinline__ bool wait_over(volatile ResWait &W, int polls) {
+    if (polls < W.spin && !W.abort) return false;
+    W.abort = 1;
+    return true;
+}
+// One thread: the block's limit at the start (iter = 0), and before the last sum of iteration `iter`.
+__device__ __forceinline__ void wait_limit(const ResComm &A, volatile ResWait &W, long long iter) {
+    if (iter == 0) {
+        W.abort = 0;
+        W.spin = A.spin;
+    }
+    if (iter == A.test_iter && (A.test_block < 0 || A.test_block == (int)blockIdx.x)) W.spin = A.test_spin;
+}
 
 // ---- tagged words -------------------------------------------------------------------------------
 __device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned tag) {
@@ -51,8 +73,8 @@ struct ResSums {
     double wsum[3][kResWarps];   // every block's partials, summed per polling warp
     CgDev cg;
     CgScalars sc;
-    int abort;                   // a wait of this block ran out
-    int left;                    // abort as the last sum left it, the same for every thread
+    ResWait wait;
+    int left;                    // wait.abort as the last sum left it, the same for every thread
 };
 
 // After p'Ap: alpha, or zero curvature (k_cg_A's test).
@@ -217,21 +239,18 @@ __device__ __forceinline__ void send_rows(const ResComm &A, const Strip<R> &S, c
 
 template <int R>
 __device__ __forceinline__ void recv_rows(const ResComm &A, const Strip<R> &S, int buf, unsigned tag, double (&s)[2],
-                                          double (&n)[2], volatile int *abort) {
+                                          double (&n)[2], volatile ResWait &W) {
     const size_t per = 2 * (size_t)(2 * A.txp);
     const uint4 *base = A.halo + (size_t)buf * A.groups * per + S.c0;
     const long blk = blockIdx.x;
     const uint4 *ps = base + (blk - 1) * (long)per + 2 * A.txp, *pn = base + (blk + 1) * (long)per;
     bool s0 = !S.south, s1 = s0, n0 = !S.north, n1 = n0;
-    for (long i = 0; !(s0 && s1 && n0 && n1); i++) {
+    for (int i = 0;; i++) {
         if (!s0) s0 = ll_try(ps, tag, s[0]);
         if (!s1) s1 = ll_try(ps + 1, tag, s[1]);
         if (!n0) n0 = ll_try(pn, tag, n[0]);
         if (!n1) n1 = ll_try(pn + 1, tag, n[1]);
-        if (i >= A.spin || *abort) {
-            if (!(s0 && s1 && n0 && n1)) *abort = 1;
-            break;
-        }
+        if ((s0 && s1 && n0 && n1) || wait_over(W, i)) break;
     }
 }
 
@@ -265,7 +284,8 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
     if (warp < 2) {
 #pragma unroll
         for (int k = 0; k < NV; k++) t[k] = sum16(sh.wred[k], lane);
-        if (warp == 0 && !alone && (int)blockIdx.x < G) {
+        // (a block whose wait ran out adds nothing: a sum that completes is one of whole partials)
+        if (warp == 0 && !alone && (int)blockIdx.x < G && !*(volatile int *)&sh.wait.abort) {
 #pragma unroll
             for (int k = 0; k < NV; k++)
                 if (lane == k) ll_store(slots + blockIdx.x * 4 + k, t[k], tag);
@@ -278,15 +298,11 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
 #pragma unroll
         for (int k = 0; k < NV; k++) x[k] = 0.0;
         if (lane < per && i < G) {
-            for (long n = 0;; n++) {
+            for (int n = 0;; n++) {
                 bool ok = true;
 #pragma unroll
                 for (int k = 0; k < NV; k++) ok = ll_try(slots + i * 4 + k, tag, x[k]) && ok;
-                if (ok) break;
-                if (n >= A.spin || *(volatile int *)&sh.abort) {
-                    *(volatile int *)&sh.abort = 1;
-                    break;
-                }
+                if (ok || wait_over(sh.wait, n)) break;
             }
         }
         __syncwarp();
@@ -303,7 +319,7 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
         }
     }
     if (warp == 0 && lane == 0) {
-        sh.left = *(volatile int *)&sh.abort;
+        sh.left = *(volatile int *)&sh.wait.abort;
         fin(t);
     }
     if (warp == 1 && lane == 0) fin2(t);

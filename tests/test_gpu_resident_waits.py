@@ -4,7 +4,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-HOOKS = ("POLLS",)
+HOOKS = ("POLLS", "BLOCK", "ITER")
 
 
 class Problem:
@@ -60,3 +60,17 @@ def test_a_block_whose_wait_ran_out_leaves_as_a_whole(shk, cuda, monkeypatch, nx
             q.solve(**kw)
     h, _ = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
     assert np.array_equal(h, want)
+
+
+@pytest.mark.parametrize("block", [0, 1, 3])
+@pytest.mark.parametrize("nx,ny,precond", [(64, 64, "chebyshev"), (200, 150, "multigrid")])
+def test_a_sum_completes_from_whole_partials_only(shk, cuda, monkeypatch, nx, ny, precond, block):
+    """One block's waits end inside the preconditioner of the last iteration, whose result enters the last
+    sums: the solve ends in an error, or with every block's rows in its norms."""
+    kw = dict(rtol=0.0, itmax=3)
+    _, ref = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
+    q = Problem(shk, monkeypatch, nx, ny, precond, POLLS=0, BLOCK=block, ITER=3)
+    for _ in range(2):
+        _, st = q.solve(**kw)
+        if st is not None:
+            assert (st.niter, st.status, st.rnorm, st.rnorm0) == (ref.niter, ref.status, ref.rnorm, ref.rnorm0)
