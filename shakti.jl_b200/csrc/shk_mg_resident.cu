@@ -48,8 +48,6 @@ struct MgResArgs : ResComm {
     double2 *vec;           // x (R = 4), in the threads' order
     const uint8_t *fmask;
     CgDev init;
-    CgDev *cg;
-    unsigned int *epoch;
     double eps_curv;
     int nd;                 // levels above the bottom ones
     MgResLevel lv[kMgResLevels];
@@ -184,14 +182,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
     __shared__ ResSums sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = A.groups, blk = blockIdx.x;
-    const unsigned tag0 = *A.epoch;  // every block reads it before the first sum; block 0 writes it after the last
-    unsigned st = tag0, vt = tag0, ht = tag0;  // tags of sums, V-cycles and row exchanges
     int rb = 0;
     volatile ResWait &W = sh.wait;
     if (tid == 0) {
         sh.cg = A.init;
         wait_limit(A, W, 0);
+        sh.tag0 = *(volatile unsigned *)A.epoch;
     }
+    __syncthreads();
+    const unsigned tag0 = sh.tag0;
+    if (tag0 == kResLost) return;  // lost before this block started
+    unsigned st = tag0, vt = tag0, ht = tag0;  // tags of sums, V-cycles and row exchanges
     auto nothing = [&]() {};
     CgScalars &sc = sh.sc;
     bool ok = true;
@@ -235,10 +236,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
                 [](double (&)[1]) {});
             if (!ok || sc.done) break;
         }
-        if (!ok && tid == 0) {
-            A.cg->fault = 1;
-            A.cg->done = 1;
-        }
+        if (!ok && tid == 0) res_end(A, tag0, kResLost, false, []() {});
         return;
     }
 
@@ -660,24 +658,16 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         }
     }
 
-    // ---- h = x + x0 -------------------------------------------------------------------------------------------
-    if (!ok) {
-        if (tid == 0) {
-            A.cg->fault = 1;
-            A.cg->done = 1;
-        }
-        return;
-    }
+    // ---- h = x + x0 (the row exchanges are the most frequent events: their tag is the last) ----------------
+    if (tid == 0) sh.kept = res_end(A, tag0, ht, ok, [&]() { *A.cg = scalars_record(sc, sh.cg); });
+    __syncthreads();
+    if (!sh.kept) return;
 #pragma unroll
     for (int j = 0; j < R; j++) {
         if (!valid(j, 0)) continue;
         const double2 xj = XG ? xg[(size_t)j * G * T] : make_double2(xr[XG ? 0 : j][0], xr[XG ? 0 : j][1]);
         A.h[cell(j, 0)] = xj.x + A.x0[cell(j, 0)];
         if (valid(j, 1)) A.h[cell(j, 1)] = xj.y + A.x0[cell(j, 1)];
-    }
-    if (blk == 0 && tid == 0) {
-        *A.cg = scalars_record(sc, sh.cg);
-        *A.epoch = ht;  // the row exchanges are the most frequent events
     }
 }
 

@@ -39,10 +39,8 @@ struct ResArgs : ResComm {
     double *h;
     const uint8_t *fmask;
     CgDev init;
-    CgDev *cg;
     ChebDev *cheb;
     double2 *vec;            // scratch vectors of the largest R, in the threads' order
-    unsigned int *epoch;     // tags used so far
     double eps_curv;
 };
 
@@ -128,16 +126,19 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     pm.g = x.g + R * x.stride;
     r.g = pm.g + R * x.stride;
     const int nx = A.nx, ny = A.ny, ty = R > 4 ? 1 : A.ty;
-    unsigned tag = *A.epoch;  // every block reads it before the first sum; block 0 writes it after the last
     int hb = 0, rb = 0, sb = 0;  // halo, sum and shared-memory buffers in turn
     if (S.tid == 0) {
         sh.cg = A.init;
         wait_limit(A, sh.wait, 0);
+        sh.tag0 = *(volatile unsigned *)A.epoch;
         if (CHEB) {
             ch.lam_min = A.cheb->lam_min;
             ch.lam_max = A.cheb->lam_max;
         }
     }
+    __syncthreads();
+    unsigned tag = sh.tag0;
+    if (tag == kResLost) return;  // lost before this block started
     auto valid = [&](int j, int e) { return S.act && S.c0 + e < nx && S.row0 + j < ny; };
     auto cell = [&](int j, int e) { return (size_t)(S.row0 + j) * nx + S.c0 + e; };
     // a / aP
@@ -427,31 +428,26 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     }
 
     // ---- h = x + x0 ----------------------------------------------------------------------------------
-    if (!ok) {
-        if (S.tid == 0) {
-            A.cg->fault = 1;
-            A.cg->done = 1;
-        }
-        return;
-    }
+    if (S.tid == 0)
+        sh.kept = res_end(A, sh.tag0, tag, ok, [&]() {
+            *A.cg = scalars_record(sc, sh.cg);
+            if (CHEB) {
+                A.cheb->est_min = ch.est_min;
+                A.cheb->est_max = ch.est_max;
+                A.cheb->adopted = ch.adopted;
+                A.cheb->lam_min = ch.lam_min;
+                A.cheb->lam_max = ch.lam_max;
+                cheb_coefficients(ch.lam_min, ch.lam_max, kMaxChebDegree, A.cheb->calpha, A.cheb->cbeta);
+            }
+        });
+    __syncthreads();
+    if (!sh.kept) return;
 #pragma unroll
     for (int j = 0; j < R; j++) {
         if (!valid(j, 0)) continue;
         const double2 xj = x.get(j);
         A.h[cell(j, 0)] = xj.x + A.x0[cell(j, 0)];
         if (valid(j, 1)) A.h[cell(j, 1)] = xj.y + A.x0[cell(j, 1)];
-    }
-    if (blockIdx.x == 0 && S.tid == 0) {
-        *A.cg = scalars_record(sc, sh.cg);
-        *A.epoch = tag;
-        if (CHEB) {
-            A.cheb->est_min = ch.est_min;
-            A.cheb->est_max = ch.est_max;
-            A.cheb->adopted = ch.adopted;
-            A.cheb->lam_min = ch.lam_min;
-            A.cheb->lam_max = ch.lam_max;
-            cheb_coefficients(ch.lam_min, ch.lam_max, kMaxChebDegree, A.cheb->calpha, A.cheb->cbeta);
-        }
     }
 }
 

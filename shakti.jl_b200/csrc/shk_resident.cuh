@@ -18,11 +18,33 @@ struct ResComm {
     int groups;              // blocks that own strips
     uint4 *red;              // [2][groups][4] tagged partials
     uint4 *halo;             // [2][groups][2][2 * txp] tagged strip-edge rows
+    CgDev *cg;
+    unsigned int *epoch;     // tags used so far, or kResLost
     int spin;                // polls before a wait gives up
     // tests: test_spin polls instead, in block test_block (-1: in every block) from the last sum of iteration
     // test_iter on (0: from the start)
     int test_spin, test_block, test_iter;
 };
+
+// A solve has one outcome, settled by the first block that swaps `epoch`: to the tags that it used when it
+// has completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here and
+// writes its rows of the head only if the solve was not lost; a block whose wait for the last sum ran out
+// when another has completed it writes them too, since it has contributed to that sum and its x is final.
+// (A sum that completes has every block's partial, so no later wait can be the one that ran out.)
+// One thread of each block; `record` is run by the one that settles a completed solve.
+constexpr unsigned kResLost = ~0u;
+template <typename Record>
+__device__ __forceinline__ bool res_end(const ResComm &A, unsigned tag0, unsigned last, bool ok, Record record) {
+    const unsigned to = ok ? last : kResLost, was = atomicCAS(A.epoch, tag0, to);
+    if (was != tag0) return was != kResLost;
+    if (ok) {
+        record();
+    } else {
+        A.cg->fault = 1;
+        A.cg->done = 1;
+    }
+    return ok;
+}
 
 // A block's waits (in its shared memory): one that runs out makes the whole block leave.
 struct ResWait {
@@ -74,6 +96,8 @@ struct ResSums {
     CgDev cg;
     CgScalars sc;
     ResWait wait;
+    unsigned tag0;               // tags used before this solve
+    int kept;                    // the solve was not lost
     int left;                    // wait.abort as the last sum left it, the same for every thread
 };
 
