@@ -590,9 +590,10 @@ SHK_API int shk_picard_solve(void *ctx, const shk_picard_opts *po, const shk_cg_
         bool deferred = false;
         rc = run_cg(c, o, &cs, &deferred);
         if (rc) return rc;
-        if (relax && (rc = launch_relax(c, po->alpha, c->h_prev))) return rc;
+        const CgDev *after = deferred ? &c->dev->cg : nullptr;
+        if (relax && (rc = launch_relax(c, po->alpha, c->h_prev, after))) return rc;
         const bool check = (iter % check_every == 0) || iter == po->iters;
-        if ((rc = launch_tail(c, check))) return rc;
+        if ((rc = launch_tail(c, check, after))) return rc;
         if ((deferred || check) && (rc = read_scalars(c))) return rc;
         if (deferred && (rc = collect_cg(c, o, &cs))) return rc;
         s.cg_iters_total += cs.niter;

@@ -295,6 +295,10 @@ static __device__ void cg_iter_finish(CgDev *cg, double rz, double rr) {
     }
 }
 
+// Work queued behind a solve whose outcome the host has not read: a solve that failed (a wait that ran out,
+// a loop that reached its bound) leaves the head and the fields as they were.  after = nullptr: no such solve.
+static __device__ __forceinline__ bool cg_ended(const CgDev *after) { return !after || (after->done && !after->fault); }
+
 // Programmatic dependent launch.  The kernels of an iteration are a chain of launches of a few us each; a
 // kernel launched by launch_after starts while the previous one of its stream still runs, as soon as all of
 // that one's blocks run, and waits here until it has completed and its writes are visible.  Every block of

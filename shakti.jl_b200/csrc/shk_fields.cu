@@ -280,15 +280,15 @@ template <bool FROM_H, bool CHECK>
 __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P, const Sliding &L,
                                           const shk_state &s, const uint8_t *__restrict__ m8,
                                           const double *__restrict__ h_prev, double *partials, unsigned int *counter,
-                                          PicDev *pic) {
+                                          PicDev *pic, bool keep = true) {
     const int lane = threadIdx.x & 31, warps = B.n * (kTailThreads / 32);
     const int nsx = (nx + kTailCols - 1) / kTailCols, per = max(1, warps / nsx), th = (ny + per - 1) / per,
               strips = nsx * ((ny + th - 1) / th);
     double red[2] = {0.0, 0.0};
     for (int st = B.id * (kTailThreads / 32) + (threadIdx.x >> 5); st < strips; st += warps) {
         const int ix = (st % nsx) * kTailCols - 1 + lane, y0 = (st / nsx) * th, y1 = min(y0 + th, ny);
-        const bool own = lane >= 1 && lane <= kTailCols && ix < nx;
-        const bool xown = own || (lane >= 1 && ix == nx);   // writes its west face (ix = nx: the domain's east edge)
+        const bool own = keep && lane >= 1 && lane <= kTailCols && ix < nx;
+        const bool xown = own || (keep && lane >= 1 && ix == nx);   // writes its west face (ix = nx: the domain's east edge)
         const bool xint = ix > 0 && ix < nx;
         // Lanes beyond the grid read the nearest cell and face, rows beyond it the last row: every load
         // is in bounds without a test, and what those lanes compute is not written.
@@ -402,8 +402,9 @@ template <bool FROM_H, bool CHECK>
 __global__ void __launch_bounds__(kTailThreads, kTailBlocksPerSm) k_tail(int nx, int ny, Params P, Sliding L, shk_state s,
                                                       const uint8_t *__restrict__ m8,
                                                       const double *__restrict__ h_prev, double *partials,
-                                                      unsigned int *counter, PicDev *pic) {
-    tail_body<FROM_H, CHECK>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic);
+                                                      unsigned int *counter, PicDev *pic, const CgDev *after) {
+    // (not a return: the flag arrives while the first rows do)
+    tail_body<FROM_H, CHECK>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic, cg_ended(after));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -515,7 +516,8 @@ __global__ void k_export_mfls(int nx, int ny, const double *aP, const double *aE
 }
 
 // relax_h! (src/elliptic_solver.jl:42-46)
-__global__ void k_relax(int n, double alpha, double *h, const double *h_prev) {
+__global__ void k_relax(int n, double alpha, double *h, const double *h_prev, const CgDev *after) {
+    if (!cg_ended(after)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         h[i] = alpha * h[i] + (1 - alpha) * h_prev[i];
 }
@@ -620,7 +622,7 @@ int launch_initial_conditions(Ctx *c) {
     c->launches++;
     if ((rc = check_launch(c, "k_init_faces"))) return rc;
     k_tail<false, false><<<tail_grid(c), kTailThreads, 0, c->stream>>>(nx, ny, c->P, c->SL, c->st, c->mask8, nullptr,
-                                                                       c->partials, c->counter, nullptr);
+                                                                       c->partials, c->counter, nullptr, nullptr);
     c->launches++;
     return check_launch(c, "k_tail<init>");
 }
@@ -647,21 +649,22 @@ int launch_export_mfls(Ctx *c, double *aP, double *aE, double *aW, double *aN, d
     return check_launch(c, "k_export_mfls");
 }
 
-int launch_tail(Ctx *c, bool picard_check) {
+int launch_tail(Ctx *c, bool picard_check, const CgDev *after) {
     if (picard_check)
         k_tail<true, true><<<tail_grid(c), kTailThreads, 0, c->stream>>>(c->nx, c->ny, c->P, c->SL, c->st, c->mask8,
                                                                         c->h_prev, c->partials, c->counter,
-                                                                        &c->dev->pic);
+                                                                        &c->dev->pic, after);
     else
         k_tail<true, false><<<tail_grid(c), kTailThreads, 0, c->stream>>>(c->nx, c->ny, c->P, c->SL, c->st, c->mask8,
-                                                                         nullptr, c->partials, c->counter, nullptr);
+                                                                         nullptr, c->partials, c->counter, nullptr,
+                                                                         after);
     c->launches++;
     return check_launch(c, "k_tail");
 }
 
-int launch_relax(Ctx *c, double alpha, const double *h_prev) {
+int launch_relax(Ctx *c, double alpha, const double *h_prev, const CgDev *after) {
     const int n = c->nx * c->ny;
-    k_relax<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, alpha, c->st.h, h_prev);
+    k_relax<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, alpha, c->st.h, h_prev, after);
     c->launches++;
     return check_launch(c, "k_relax");
 }

@@ -259,8 +259,9 @@ int mg_set_first_wait_polls();
 int launch_initial_conditions(Ctx *c);
 int launch_assemble(Ctx *c, int parabolic, double dt, bool copy_h_prev);
 int launch_export_mfls(Ctx *c, double *aP, double *aE, double *aW, double *aN, double *aS, double *rhs);
-int launch_tail(Ctx *c, bool picard_check);
-int launch_relax(Ctx *c, double alpha, const double *h_prev);
+// after: the solve these follow without the host having read its outcome (cg_ended), or nullptr
+int launch_tail(Ctx *c, bool picard_check, const CgDev *after = nullptr);
+int launch_relax(Ctx *c, double alpha, const double *h_prev, const CgDev *after = nullptr);
 int launch_step_b(Ctx *c, double dt);
 int launch_fill(Ctx *c, double *dst, double v, size_t n);
 int launch_fill_plus_base(Ctx *c, double *dst, double v, const double *base, size_t n);

@@ -379,12 +379,15 @@ __global__ void __launch_bounds__(kThreads) k_cg_B(int n, const T *__restrict__ 
 __device__ __forceinline__ void cg_finish_body(Blk B, int n, const double *x, double *h) {
     for (int i = B.id * blockDim.x + threadIdx.x; i < n; i += B.n * blockDim.x) h[i] = x[i] + h[i];
 }
-__global__ void k_cg_finish(int n, const double *x, double *h) { cg_finish_body(grid_blk(), n, x, h); }
+__global__ void k_cg_finish(int n, const double *x, double *h, const CgDev *cg) {
+    if (cg_ended(cg)) cg_finish_body(grid_blk(), n, x, h);
+}
 // Multigrid form: h = x + x0 with the x update that the last iteration left pending (CgDev::x_pending;
 // the rounding of the single update).  One pass where the update and the addition took two (60 and
 // 66 us at 4096^2).
 __global__ void k_cg_finish_mg(int n, const double *x, const double *x0, double *h, const double *p0, const double *p1,
                                const CgDev *cg) {
+    if (!cg_ended(cg)) return;
     const int pend = cg->x_pending;
     const double *p = pend == 1 ? p0 : p1;
     const double a = cg->alpha;
@@ -395,7 +398,8 @@ __global__ void k_cg_finish_mg(int n, const double *x, const double *x0, double 
     }
 }
 // h = x + x0 for a warm start x0 other than h
-__global__ void k_cg_finish_from(int n, const double *x, const double *x0, double *h) {
+__global__ void k_cg_finish_from(int n, const double *x, const double *x0, double *h, const CgDev *cg) {
+    if (!cg_ended(cg)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) h[i] = x[i] + x0[i];
 }
 
@@ -1169,9 +1173,9 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
             k_cg_finish_mg<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, x0, c->st.h, c->p[0], c->p[1],
                                                                         &c->dev->cg);
         else if (x0 == c->st.h)
-            k_cg_finish<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, c->st.h);
+            k_cg_finish<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, c->st.h, &c->dev->cg);
         else
-            k_cg_finish_from<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, x0, c->st.h);
+            k_cg_finish_from<<<flat_grid(c, n), kThreads, 0, c->stream>>>(n, c->x, x0, c->st.h, &c->dev->cg);
         c->launches++;
         if ((rc = check_launch(c, "cg finish"))) return rc;
         if (deferred) {
@@ -1562,7 +1566,7 @@ extern "C" SHK_API int shk_cg_solve_static(int nx, int ny, const double *aP, con
         if (cudaGetLastError() != cudaSuccess) return SHK_CUDA_ERROR;
         if (batch < 256) batch *= 2;
     }
-    k_cg_finish<<<std::max(1, std::min(sms * 8, (n + kThreads - 1) / kThreads)), kThreads, 0, s>>>(n, xc, x);
+    k_cg_finish<<<std::max(1, std::min(sms * 8, (n + kThreads - 1) / kThreads)), kThreads, 0, s>>>(n, xc, x, nullptr);
     if (cudaGetLastError() != cudaSuccess) return SHK_CUDA_ERROR;
     if (cudaMemcpyAsync(&h, cg, sizeof(CgDev), cudaMemcpyDeviceToHost, s) != cudaSuccess) return SHK_CUDA_ERROR;
     if (cudaStreamSynchronize(s) != cudaSuccess) return SHK_CUDA_ERROR;

@@ -90,3 +90,17 @@ def test_a_solve_has_one_outcome(shk, cuda, monkeypatch, nx, ny, precond, block)
             assert np.array_equal(h, q.h0.cpu().numpy())
         else:
             assert np.array_equal(h, want) and (st.niter, st.rnorm) == (ref.niter, ref.rnorm)
+
+
+@pytest.mark.parametrize("alpha", [None, 0.7])
+@pytest.mark.parametrize("nx,ny,precond", [(201, 150, "jacobi"), (64, 64, "chebyshev"), (200, 150, "multigrid")])
+def test_a_failed_solve_leaves_the_fields(shk, cuda, monkeypatch, nx, ny, precond, alpha):
+    """The Picard loop queues head relaxation and the field update behind a solve before it knows the
+    outcome: after a solve that failed neither has written anything."""
+    q = Problem(shk, monkeypatch, nx, ny, precond, POLLS=0)
+    before = {f: q.s[f].clone() for f in shk._lib.STATE_FIELDS}
+    ps = shk.PicardSolver(5, 1e-6, q.solver(rtol=1e-10), q.g, alpha=alpha)
+    with pytest.raises(shk._lib.ShaktiError, match="did not complete"):
+        shk.Picard_loop(ps, q.s, q.g, q.p, None, shk.Arithmetic(), q.sl)
+    for f, t in before.items():
+        assert cuda.equal(q.s[f], t), f
