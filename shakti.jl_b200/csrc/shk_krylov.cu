@@ -1118,6 +1118,7 @@ int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
 // scalars after the work it queues next and calls collect_cg.
 int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
     if (deferred) *deferred = false;
+    c->loop_trip_launches = 0;  // (left by a solve whose outcome was never collected)
     const int nx = c->nx, ny = c->ny, n = nx * ny;
     const double *ws = c->ws_x0;  // consumed by this solve (Float64 forms; ignored by the mixed form)
     c->ws_x0 = nullptr;
