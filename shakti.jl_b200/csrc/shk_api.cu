@@ -315,6 +315,7 @@ SHK_API int shk_create(int nx, int ny, double lx, double ly, void *stream, void 
     // tests of the resident solves' waits (ResComm): their limit, in one block, from one iteration on
     if (const char *v = getenv("SHK_TEST_RESIDENT_POLLS")) c->res_test_spin = std::max(0, atoi(v));
     if (const char *v = getenv("SHK_TEST_RESIDENT_BLOCK")) c->res_test_block = atoi(v);
+    if (const char *v = getenv("SHK_TEST_RESIDENT_ABSENT")) c->res_test_absent = atoi(v);
     if (const char *v = getenv("SHK_TEST_RESIDENT_ITER")) c->res_test_iter = std::max(0, atoi(v));
     c->max_blocks = c->grid_stencil > c->march_blocks ? c->grid_stencil : c->march_blocks;
     if (c->max_blocks < c->num_sms * 8) c->max_blocks = c->num_sms * 8;
@@ -587,15 +588,19 @@ SHK_API int shk_picard_solve(void *ctx, const shk_picard_opts *po, const shk_cg_
         c->assembled_parabolic = false;
         shk_cg_stats cs;
         memset(&cs, 0, sizeof(cs));
-        bool deferred = false;
-        rc = run_cg(c, o, &cs, &deferred);
-        if (rc) return rc;
-        const CgDev *after = deferred ? &c->dev->cg : nullptr;
-        if (relax && (rc = launch_relax(c, po->alpha, c->h_prev, after))) return rc;
         const bool check = (iter % check_every == 0) || iter == po->iters;
-        if ((rc = launch_tail(c, check, after))) return rc;
-        if ((deferred || check) && (rc = read_scalars(c))) return rc;
-        if (deferred && (rc = collect_cg(c, o, &cs))) return rc;
+        for (bool resident = true;; resident = false) {
+            bool deferred = false;
+            if ((rc = run_cg(c, o, &cs, &deferred, resident))) return rc;
+            const CgDev *after = deferred ? &c->dev->cg : nullptr;
+            if (relax && (rc = launch_relax(c, po->alpha, c->h_prev, after))) return rc;
+            if ((rc = launch_tail(c, check, after))) return rc;
+            if ((deferred || check) && (rc = read_scalars(c))) return rc;
+            if (!deferred) break;
+            rc = collect_cg(c, o, &cs);
+            if (rc == SHK_OK) break;
+            if (rc != kNotStarted) return rc;
+        }
         s.cg_iters_total += cs.niter;
         s.cg_solves++;
         if (cs.status == SHK_BREAKDOWN) s.cg_breakdowns++;

@@ -56,7 +56,7 @@ struct CgDev {
     int done, status, first, stop_rule;
     int cont;        // init continues the previous search direction instead of restarting
     unsigned int trips;  // trips of the device-side iteration loop (bounded)
-    int fault;           // set by a kernel whose bounded wait for a tile copy ran out
+    int fault;           // kFault...: a bounded wait ran out
     // paired x updates of the multigrid form: alpha of the previous iteration, and which search
     // direction's x update is still to be applied (0 none, 1 + the p buffer's index)
     double alpha_prev;
@@ -84,8 +84,14 @@ struct DevScalars {
     PicDev pic;
     double ref_rr, ref_bb; // mixed precision: outer residual norms
     unsigned int res_epoch; // resident solve: exchange tags used so far
-    unsigned int pad;
+    unsigned int res_arrived; // blocks of the resident solve that have started
 };
+
+// CgDev::fault: a tile copy or an exchange did not arrive; not every block of a resident solve started in
+// time.  The second is no failure of the solve: it ends as kNotStarted (as does a refused launch), and the
+// general kernels take its place.
+constexpr int kFaultWait = 1, kFaultNotStarted = 2;
+constexpr int kNotStarted = -1000;
 
 // Geometry of the resident solve (shk_resident.cu): rows per thread, threads per row group, row
 // groups per block, blocks (0: the grid does not fit).
@@ -178,7 +184,10 @@ struct Ctx {
     uint4 *res_red = nullptr, *res_halo = nullptr;  // its exchange buffers
     double2 *res_vec = nullptr;                     // its scratch vectors
     bool res_restart = false; // its tags start over at the next solve
-    int res_spin = 1 << 21;   // polls before one of its waits gives up
+    int res_spin = 1 << 21;   // polls before one of its waits gives up (about 1 s)
+    int res_start_spin = 1 << 16;           // and before it gives up on blocks that have not started (about 40 ms)
+    int res_test_absent = -1;               // tests: ResComm's
+    const double *res_ws = nullptr;         // the warm start of the last resident solve
     int res_test_spin = -1, res_test_block = -1, res_test_iter = 0; // tests: ResComm's (-1: none)
     int max_blocks = 0;
     int grid_stencil = 0;    // blocks for tile-stride kernels
@@ -271,7 +280,7 @@ int launch_matvec(Ctx *c, const double *x, double *y);
 int run_chebyshev_bounds(Ctx *c, int nsteps, const double *rhs);
 int cheb_set_bounds(Ctx *c, double lmin, double lmax);
 int launch_chebyshev_apply_standalone(Ctx *c, int degree, const double *x, double *y);
-int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred = nullptr);
+int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred = nullptr, bool resident = true);
 int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st);
 int read_scalars(Ctx *c);
 int move_scalars(Ctx *c, void *dst, const void *src, size_t bytes, bool to_host);
@@ -286,7 +295,8 @@ size_t res_vec_bytes(const ResPlan &P);
 bool res_serves(const Ctx *c, const shk_cg_opts *o);
 int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0);
 int res_tags(Ctx *c);
-void res_waits(const Ctx *c, struct ResComm &a);
+void res_waits(Ctx *c, struct ResComm &a);
+int res_cooperative(Ctx *c, const void *kernel, int blocks, void *args, size_t smem, const char *what);
 
 // shk_mg_resident.cu
 void mg_res_plan(Ctx *c);

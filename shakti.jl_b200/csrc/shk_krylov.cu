@@ -1090,11 +1090,16 @@ static int cg_core(Ctx *c, const shk_cg_opts *o, CgDev *cgd, CgDev *cgh, const T
     return SHK_OK;
 }
 
-// A Float64 solve's outcome from the scalars last read back.
+// A Float64 solve's outcome from the scalars last read back; kNotStarted: a resident solve that has not begun
+// (the caller runs it without `resident`).
 int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
     const CgDev &g = c->host_dev->cg;
     if (g.fault) {
         c->res_restart = true;
+        if (g.fault == kFaultNotStarted) {
+            c->ws_x0 = c->res_ws;
+            return kNotStarted;
+        }
         return fail(c, SHK_CUDA_ERROR, res_serves(c, o) || mg_res_serves(c, o)
                                            ? "an exchange of the resident solve did not complete (bounded wait ran out)"
                                            : "a TMA tile copy did not complete (bounded wait ran out)");
@@ -1116,7 +1121,7 @@ int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
 
 // With `deferred`, a solve may return before it has finished (*deferred set): the caller reads the
 // scalars after the work it queues next and calls collect_cg.
-int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
+int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred, bool resident) {
     if (deferred) *deferred = false;
     c->loop_trip_launches = 0;  // (left by a solve whose outcome was never collected)
     const int nx = c->nx, ny = c->ny, n = nx * ny;
@@ -1142,17 +1147,21 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred) {
             return fail(c, SHK_BAD_ARG, "chebyshev nsteps must be in [2, 64]");
     }
     // the whole solve in one persistent kernel where the grid's Krylov state fits on the chip
-    if (res_serves(c, o) || mg_res_serves(c, o)) {
+    if (resident && (res_serves(c, o) || mg_res_serves(c, o))) {
         const CgDev init = make_cg_init(o, n, false, 0.0);
         const double *x0 = ws ? ws : c->st.h;
+        c->res_ws = ws;
         int rc = mg_res_serves(c, o) ? mg_res_solve(c, init, x0) : res_solve(c, o, init, x0);
-        if (rc) return rc;
-        if (deferred) {
-            *deferred = true;
-            return SHK_OK;
+        if (rc == SHK_OK) {
+            if (deferred) {
+                *deferred = true;
+                return SHK_OK;
+            }
+            if ((rc = read_scalars(c))) return rc;
+            rc = collect_cg(c, o, st);
+            c->ws_x0 = nullptr;
         }
-        if ((rc = read_scalars(c))) return rc;
-        return collect_cg(c, o, st);
+        if (rc != kNotStarted) return rc;
     }
     if (o->precond == SHK_PRECOND_CHEBYSHEV) {
         // _cg_precond! refreshes the bounds from this solve's rhs (src/linear_solver.jl:853-856)

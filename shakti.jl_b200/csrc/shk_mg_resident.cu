@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
     if (tid == 0) {
         sh.cg = A.init;
         wait_limit(A, W, 0);
-        sh.tag0 = *(volatile unsigned *)A.epoch;
+        sh.tag0 = res_arrive(A);
     }
     __syncthreads();
     const unsigned tag0 = sh.tag0;
@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         BotShared &M = *reinterpret_cast<BotShared *>(smem);
         BotOp O;
         bot_load(A.bp, M, O);
+        if (tid == 0) sh.kept = res_started(A, tag0);
         __syncthreads();
+        if (!sh.kept) return;
         double v3[3] = {0.0, 0.0, 0.0}, v1[1] = {0.0}, v2[2] = {0.0, 0.0};
         for (bool first = true;; first = false) {  // (one place for the V-cycle: its registers stay registers)
             vt++;
@@ -307,6 +309,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         for (int x = tid; x < M.nx; x += T) M.N[x] = M.y0 > 0 ? V.aN[(size_t)(M.y0 - 1) * M.nx + x] : 0.0f;
         for (int i = tid; i < 2 * (M.n + 2 * M.nx); i += T) M.X0[i] = 0.0f;
     }
+
+    if (tid == 0) sh.kept = res_started(A, tag0);
+    __syncthreads();
+    if (!sh.kept) return;
 
     double r[R][2], p[R][2], q[R][2], xr[XG ? 1 : R][2];
     double rs[2] = {0.0, 0.0}, rn[2] = {0.0, 0.0};  // r on the rows below and above the strip
@@ -725,14 +731,7 @@ size_t mg_res_vec_bytes(const Ctx *c) {
 
 template <int R>
 static int mg_res_launch(Ctx *c, MgResArgs &a, size_t smem) {
-    auto kernel = k_mg_resident<R>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return check_cuda(c, e, "resident multigrid solve shared memory");
-    void *args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(c->mg_res.blocks + 1), dim3(kResThreads), args, smem,
-                                    c->stream);
-    c->launches++;
-    return check_cuda(c, e, "resident multigrid solve launch");
+    return res_cooperative(c, (const void *)k_mg_resident<R>, c->mg_res.blocks + 1, &a, smem, "resident multigrid solve launch");
 }
 
 bool mg_res_serves(const Ctx *c, const shk_cg_opts *o) {
@@ -788,8 +787,6 @@ int mg_res_solve(Ctx *c, const CgDev &init, const double *x0) {
     a.vec = c->mg_res_vec;
     a.fmask = c->mask8;
     a.init = init;
-    a.cg = &c->dev->cg;
-    a.epoch = &c->dev->res_epoch;
     a.eps_curv = DBL_EPSILON;
     a.wc = c->mg_omega_c;
     const size_t smem = mg_res_smem(c, P.rows, P.txp, P.ty, a.nd, a.lv);

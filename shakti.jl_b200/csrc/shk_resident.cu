@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     if (S.tid == 0) {
         sh.cg = A.init;
         wait_limit(A, sh.wait, 0);
-        sh.tag0 = *(volatile unsigned *)A.epoch;
+        sh.tag0 = res_arrive(A);
         if (CHEB) {
             ch.lam_min = A.cheb->lam_min;
             ch.lam_max = A.cheb->lam_max;
@@ -175,6 +175,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
         }
     S.aS0 = S.row0 > 0 && valid(0, 0) ? A.aN[cell(-1, 0)] : 0.0;
     S.aS1 = S.row0 > 0 && valid(0, 1) ? A.aN[cell(-1, 1)] : 0.0;
+    if (S.tid == 0) sh.kept = res_started(A, sh.tag0);
+    __syncthreads();
+    if (!sh.kept) return;
     // v on the thread's rows -> the operator's inputs around it (block barrier inside)
     auto share = [&](const double (&v)[R][2], double (&s)[2], double (&n)[2]) {
         if (CHEB) sb ^= 1;
@@ -685,16 +688,25 @@ size_t res_vec_bytes(const ResPlan &P) {
 }
 size_t res_halo_bytes(const ResPlan &P) { return (size_t)2 * P.blocks * 2 * (2 * P.txp) * sizeof(uint4); }
 
-template <int R, bool CHEB>
-static int res_launch(Ctx *c, ResArgs &a) {  // a cooperative launch: every block is resident
-    constexpr size_t smem = ResSmem<R, CHEB>::bytes;
-    auto kernel = k_cg_resident<R, CHEB>;
+// A cooperative launch: the blocks run together, or not at all.  On a part of the device too small for them
+// (a green context, an MPS share) it is refused, and the general kernels serve.
+int res_cooperative(Ctx *c, const void *kernel, int blocks, void *args, size_t smem, const char *what) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return check_cuda(c, e, "resident solve shared memory");
-    void *args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(c->res[CHEB].blocks), dim3(kResThreads), args, smem, c->stream);
+    if (e != cudaSuccess) return check_cuda(c, e, what);
+    void *list[] = {args};
+    e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kResThreads), list, smem, c->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kNotStarted;
+    }
     c->launches++;
-    return check_cuda(c, e, "resident solve launch");
+    return check_cuda(c, e, what);
+}
+
+template <int R, bool CHEB>
+static int res_launch(Ctx *c, ResArgs &a) {
+    return res_cooperative(c, (const void *)k_cg_resident<R, CHEB>, c->res[CHEB].blocks, &a, ResSmem<R, CHEB>::bytes,
+                           "resident solve launch");
 }
 
 template <bool CHEB>
@@ -712,17 +724,22 @@ bool res_serves(const Ctx *c, const shk_cg_opts *o) {
                                         (o->precond == SHK_PRECOND_CHEBYSHEV && c->res[1].blocks > 0));
 }
 
-// Tags are 32 bits wide: start over long before they could repeat (and after a fault).
+// Tags have 31 bits: start over long before they could repeat (and after a lost solve).
 int res_tags(Ctx *c) {
-    if (!c->res_restart && c->host_dev->res_epoch <= (1u << 31)) return SHK_OK;
+    if (!c->res_restart && c->host_dev->res_epoch <= (1u << 30)) return SHK_OK;
     cudaError_t e = cudaMemsetAsync(c->res_comm, 0, c->res_comm_bytes, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&c->dev->res_epoch, 0, sizeof(unsigned int), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->dev->res_epoch, 0, 2 * sizeof(unsigned int), c->stream);  // and res_arrived
     c->res_restart = false;
     return check_cuda(c, e, "resident solve buffers");
 }
 
-void res_waits(const Ctx *c, ResComm &a) {
+void res_waits(Ctx *c, ResComm &a) {
+    a.cg = &c->dev->cg;
+    a.epoch = &c->dev->res_epoch;
+    a.arrived = &c->dev->res_arrived;
     a.spin = c->res_spin;
+    a.start_spin = c->res_start_spin;
+    a.test_absent = c->res_test_absent;
     a.test_spin = c->res_test_spin;
     a.test_block = c->res_test_block;
     a.test_iter = c->res_test_spin < 0 ? -1 : c->res_test_iter;
@@ -759,11 +776,9 @@ int res_solve(Ctx *c, const shk_cg_opts *o, const CgDev &init, const double *x0)
     a.vec = c->res_vec;
     a.fmask = c->mask8;
     a.init = init;
-    a.cg = &c->dev->cg;
     a.cheb = &c->dev->cheb;
     a.red = c->res_red;
     a.halo = c->res_halo;
-    a.epoch = &c->dev->res_epoch;
     a.eps_curv = DBL_EPSILON;
     res_waits(c, a);
     return cheb ? res_launch_rows<true>(c, a) : res_launch_rows<false>(c, a);

@@ -19,28 +19,67 @@ struct ResComm {
     uint4 *red;              // [2][groups][4] tagged partials
     uint4 *halo;             // [2][groups][2][2 * txp] tagged strip-edge rows
     CgDev *cg;
-    unsigned int *epoch;     // tags used so far, or kResLost
+    unsigned int *epoch;     // tags used so far: the solve's word (res_arrive)
+    unsigned int *arrived;   // blocks that have started
     int spin;                // polls before a wait gives up
+    int start_spin;          // polls before a block stops waiting for the launch's other blocks to start
     // tests: test_spin polls instead, in block test_block (-1: in every block) from the last sum of iteration
     // test_iter on (0: from the start)
     int test_spin, test_block, test_iter;
+    int test_absent;         // tests: this block does not start (-1: none)
 };
 
-// A solve has one outcome, settled by the first block that swaps `epoch`: to the tags that it used when it
-// has completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here and
+// A solve's word, `epoch`, moves on by compare-and-swap only, so every block sees the same solve:
+//   t             t tags used so far, no solve running (t < kResRunning: res_tags)
+//   kResRunning|t every block of the solve that found t has started
+//   t' > t        completed, the tags up to t' used
+//   kResLost      lost: not every block started in time, or a wait ran out
+constexpr unsigned kResRunning = 1u << 31, kResLost = ~0u;
+
+// Starting.  The blocks of a cooperative launch run together, but not from the same moment: another stream's
+// kernel may hold some of their SMs for as long as it likes.  So no block polls for another's words before all
+// of them have started, and when that takes too long (start_spin) the solve is lost before it began and the
+// host turns to the general kernels, whose blocks wait for nobody.  The last block to arrive starts the
+// solve; the blocks load their operator meanwhile.  One thread of each block calls these.
+__device__ __forceinline__ unsigned res_arrive(const ResComm &A) {  // returns t, or kResLost
+    const unsigned t = *(volatile unsigned *)A.epoch;
+    if (t == kResLost || A.test_absent == (int)blockIdx.x) return kResLost;
+    __threadfence();
+    if (atomicAdd(A.arrived, 1u) + 1 == gridDim.x) {
+        *(volatile unsigned *)A.arrived = 0;
+        __threadfence();
+        atomicCAS(A.epoch, t, t | kResRunning);
+    }
+    return t;
+}
+__device__ __forceinline__ bool res_started(const ResComm &A, unsigned t) {
+    for (int i = 0;; i++) {
+        const unsigned w = *(volatile unsigned *)A.epoch;
+        if (w != t) return w == (t | kResRunning);
+        if (i < A.start_spin) continue;
+        const unsigned was = atomicCAS(A.epoch, t, kResLost);
+        if (was == t) {
+            A.cg->fault = kFaultNotStarted;
+            A.cg->done = 1;
+        }
+        return was == (t | kResRunning);
+    }
+}
+
+// Ending.  The outcome is settled by the first block that swaps the word: to the tags that it used when it has
+// completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here and
 // writes its rows of the head only if the solve was not lost; a block whose wait for the last sum ran out
 // when another has completed it writes them too, since it has contributed to that sum and its x is final.
 // (A sum that completes has every block's partial, so no later wait can be the one that ran out.)
-// One thread of each block; `record` is run by the one that settles a completed solve.
-constexpr unsigned kResLost = ~0u;
+// `record` is run by the one that settles a completed solve.
 template <typename Record>
-__device__ __forceinline__ bool res_end(const ResComm &A, unsigned tag0, unsigned last, bool ok, Record record) {
-    const unsigned to = ok ? last : kResLost, was = atomicCAS(A.epoch, tag0, to);
-    if (was != tag0) return was != kResLost;
+__device__ __forceinline__ bool res_end(const ResComm &A, unsigned t, unsigned last, bool ok, Record record) {
+    const unsigned to = ok ? last : kResLost, was = atomicCAS(A.epoch, t | kResRunning, to);
+    if (was != (t | kResRunning)) return was != kResLost;
     if (ok) {
         record();
     } else {
-        A.cg->fault = 1;
+        A.cg->fault = kFaultWait;
         A.cg->done = 1;
     }
     return ok;
@@ -97,7 +136,7 @@ struct ResSums {
     CgScalars sc;
     ResWait wait;
     unsigned tag0;               // tags used before this solve
-    int kept;                    // the solve was not lost
+    int kept;                    // the solve has started; at the end: it was not lost
     int left;                    // wait.abort as the last sum left it, the same for every thread
 };
 

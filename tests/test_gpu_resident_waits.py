@@ -4,7 +4,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-HOOKS = ("POLLS", "BLOCK", "ITER")
+HOOKS = ("POLLS", "BLOCK", "ITER", "ABSENT")
 
 
 class Problem:
@@ -104,3 +104,59 @@ def test_a_failed_solve_leaves_the_fields(shk, cuda, monkeypatch, nx, ny, precon
         shk.Picard_loop(ps, q.s, q.g, q.p, None, shk.Arithmetic(), q.sl)
     for f, t in before.items():
         assert cuda.equal(q.s[f], t), f
+
+
+@pytest.mark.parametrize("block", [0, 2])
+@pytest.mark.parametrize("nx,ny,precond", FORMS)
+def test_a_solve_that_cannot_start_runs_by_the_general_kernels(shk, cuda, monkeypatch, nx, ny, precond, block):
+    """A block of the launch that does not start (another stream's kernel holds its SM): the same head, bit
+    for bit, as by the general kernels, and no error; in the Picard loop too, where the warm start and
+    the relaxation come after it."""
+    out = []
+    for resident, hooks in ((False, {}), (True, dict(ABSENT=block))):
+        q = Problem(shk, monkeypatch, nx, ny, precond, resident=resident, **hooks)
+        h, st = q.solve(rtol=1e-10)
+        ps = shk.PicardSolver(2, 1e-30, q.solver(rtol=1e-8), q.g, alpha=0.7)
+        q.s.h.copy_(q.h0)
+        shk.Picard_loop(ps, q.s, q.g, q.p, None, shk.Arithmetic(), q.sl)
+        out.append((h, st.niter, st.status, st.rnorm, ps.cg_iters_total, {f: q.s[f].clone() for f in shk._lib.STATE_FIELDS}))
+    a, b = out
+    assert np.array_equal(a[0], b[0]) and a[1:5] == b[1:5] and a[2] == 0
+    for f, t in a[5].items():
+        assert cuda.equal(b[5][f], t), f
+
+
+def test_two_solves_at_once(shk, cuda, monkeypatch):
+    """Two host threads on two streams: each gets its own solution, whether the two launches follow one
+    another or one gives way to the general kernels (to 1e-9, as between the two forms)."""
+    from concurrent.futures import ThreadPoolExecutor
+    forms = [(640, 300, "jacobi"), (385, 301, "multigrid")]
+    want = [Problem(shk, monkeypatch, *f).solve(rtol=1e-11)[0] for f in forms]
+    qs = []
+    for f in forms:
+        stream = cuda.cuda.Stream()
+        with cuda.cuda.stream(stream):
+            qs.append((stream, Problem(shk, monkeypatch, *f)))
+    cuda.cuda.synchronize()
+
+    def work(k):
+        stream, q = qs[k]
+        with cuda.cuda.stream(stream):
+            return [q.solve(rtol=1e-11) for _ in range(20)]
+    with ThreadPoolExecutor(2) as ex:
+        runs = list(ex.map(work, range(2)))
+    for k, run in enumerate(runs):
+        for h, st in run:
+            assert st is not None and st.status == 0
+            assert np.max(np.abs(h - want[k])) <= 1e-9 * np.max(np.abs(want[k]))
+
+
+@pytest.mark.parametrize("nx,ny,precond", [(640, 300, "jacobi"), (513, 301, "chebyshev"), (385, 301, "multigrid")])
+def test_a_part_of_the_device(shk, cuda, monkeypatch, nx, ny, precond):
+    """A stream on 16 SMs, too few for the launch's blocks: the general kernels' head, bit for bit."""
+    kw = dict(rtol=0.0, itmax=20)
+    want, ref = Problem(shk, monkeypatch, nx, ny, precond, resident=False).solve(**kw)
+    part = cuda.cuda.GreenContext.create(16, 0)
+    with cuda.cuda.stream(part.Stream()):
+        h, st = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
+    assert (st.niter, st.status) == (ref.niter, ref.status) and np.array_equal(h, want)
