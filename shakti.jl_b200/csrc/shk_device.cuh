@@ -69,7 +69,7 @@ __device__ __forceinline__ double quotient(double a, double d, double y) {
 }
 __device__ __forceinline__ double quotient_any(double a, double d, double y) {
     const double t = a * y, c = fma(fma(-d, t, a), y, t);
-    return isinf(t) ? t : c;
+    return (__double2hiint(t) & 0x7ff00000) == 0x7ff00000 ? t : c;  // infinite or NaN: t
 }
 
 // ---- tiles -------------------------------------------------------------------------------------

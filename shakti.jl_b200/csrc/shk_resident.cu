@@ -141,11 +141,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     if (tag == kResLost) return;  // lost before this block started
     auto valid = [&](int j, int e) { return S.act && S.c0 + e < nx && S.row0 + j < ny; };
     auto cell = [&](int j, int e) { return (size_t)(S.row0 + j) * nx + S.c0 + e; };
-    // a / aP
-    auto over_aP = [&](double a, int j, int e) {
+    // a / aP; r / aP keeps an infinite r (after an operator application an infinite value ends in NaN anyway)
+    auto over_aP = [&](double a, int j, int e, bool residual = false) {
         const double d = sm[(2 * j + e) * T + S.tid];
         if (j < L::recip) {
-            return quotient(a, d, sm[(6 * R + 2 * j + e) * T + S.tid]);
+            const double y = sm[(6 * R + 2 * j + e) * T + S.tid];
+            return residual ? quotient_any(a, d, y) : quotient(a, d, y);
         }
         const bool zero = a == 0.0 && d > 0.0 && d < INFINITY;
         const double c = (zero ? d : a) / d;
@@ -285,8 +286,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
                 const double2 rj = r.get(j);
                 const double r0 = rj.x + f * q[j][0], r1 = rj.y + f * q[j][1];
                 r.set(j, r0, r1);
-                q[j][0] = over_aP(r0, j, 0);
-                q[j][1] = over_aP(r1, j, 1);
+                q[j][0] = over_aP(r0, j, 0, true);
+                q[j][1] = over_aP(r1, j, 1, true);
                 v[0] += r0 * q[j][0];
                 v0 += r1 * q[j][1];
                 v[1] += r0 * r0;
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 if (L::pmode == V_REG) pk[CHEB ? j : 0][e] = w1[j][e];
-                w1[j][e] = over_aP(rv[e], j, e);
+                w1[j][e] = over_aP(rv[e], j, e, true);
                 rc[j][e] = w1[j][e];
                 q[j][e] = 0.0 + a * w1[j][e];
             }
@@ -562,7 +563,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_cg_tiny(const __grid_consta
     __syncthreads();  // every r is read: Z takes z
 #pragma unroll
     for (int k = 0; k < 5; k++)
-        if (has[k]) Z[cell[k]] = quotient(r[k], D[cell[k]], inv[k]);
+        if (has[k]) Z[cell[k]] = quotient_any(r[k], D[cell[k]], inv[k]);
     __syncthreads();
     const int nbA = (ny + kTinyRows - 1) / kTinyRows;
     while (!sc.done) {
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_cg_tiny(const __grid_consta
             const int c = cell[k];
             x[k] = x[k] + alpha * Pv[c];
             r[k] = r[k] + (-alpha) * Q[c];
-            const double z = quotient(r[k], D[c], inv[k]);
+            const double z = quotient_any(r[k], D[c], inv[k]);
             Z[c] = z;
             v[0] += r[k] * z;
             v[1] += r[k] * r[k];
