@@ -161,8 +161,9 @@ __device__ __forceinline__ double taub_face(const Params &P, const Sliding &L, d
     if (L.kind == SHK_SLIDING_LINEAR) return Cf * Nf * ub;
     if (!(abs_v > 0)) return 0.0;
     double denom = (L.kind == SHK_SLIDING_REG_COULOMB_V0) ? L.v0 : jl_pow(fabs(Nf), P.n, P.n_int) * lf;
-    // no sliding across this face: the drag is 0 (with its sign), whatever the root below
-    if (ub == 0.0 && abs_v < INFINITY && denom == denom) return Nf * Cf * ub;
+    // no sliding across this face: the drag is 0 (with its sign) where the root below is finite, which a
+    // ratio in [0, 1] gives (a negative denominator, from v0 < 0 or lambda < 0, may give NaN or infinity)
+    if (ub == 0.0 && abs_v < INFINITY && denom >= 0) return Nf * Cf * ub;
     // x^(1/n): for n = 3, cbrt (a fraction of pow's cost; it differs from pow(x, 1/3.0) by at most
     // about an ulp, within the tolerance the parity tests hold the pow-dependent fields to)
     const double ratio = abs_v / (abs_v + denom);
