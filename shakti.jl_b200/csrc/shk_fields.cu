@@ -212,12 +212,20 @@ __device__ __forceinline__ CellQ make_cell(const Params &P, const CellRaw &r) {
 struct FaceRaw {
     double valid, b, ub;
 };
+// Where a law keeps its face coefficients, or the prescribed drag (nullptr: one coefficient for all faces).
+// They are requested with a row's first loads: fetched where the drag is formed, after the square root, they
+// were one more wait per face (3000 x 3000, v0 law: 659 us; 769 so, and 715 before the warps marched).
+template <int DIR>
+__device__ __forceinline__ const double *face_coef(const Sliding &L, const shk_state &s) {
+    if (L.kind == SHK_SLIDING_PRESCRIBED) return DIR == 0 ? s.taub_x : s.taub_y;
+    return L.kind == SHK_SLIDING_REG_COULOMB ? nullptr : (DIR == 0 ? L.Cx : L.Cy);
+}
 
 // x- (DIR 0) or y-face (DIR 1) between cells a (west/south) and b (east/north); a or b may be absent
 // at the domain edge (edge face: gradients read from memory, taub uses the one adjacent cell).
 template <bool FROM_H, int DIR>
 __device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const shk_state &s, unsigned fi, bool interior, const CellQ &a, const CellQ &b, const CellQ &edge_cell,
-                                        const FaceRaw &r) {
+                                        const FaceRaw &r, double Cf) {
     FaceOut o;
     if (interior && FROM_H) {
         const double dd = DIR == 0 ? P.dx : P.dy, inv = DIR == 0 ? P.dx_inv : P.dy_inv;
@@ -230,7 +238,7 @@ __device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const
     q_re(P, r.b, o.dh, o.q, o.re);
     o.ub = r.ub;
     if (L.kind == SHK_SLIDING_PRESCRIBED) {
-        o.taub = (DIR == 0 ? s.taub_x : s.taub_y)[fi];
+        o.taub = Cf;
     } else {
         double Nf, lf, av;
         if (interior) {
@@ -242,7 +250,6 @@ __device__ __forceinline__ FaceOut face(const Params &P, const Sliding &L, const
             lf = edge_cell.lam;
             av = edge_cell.aub;
         }
-        const double Cf = (L.kind == SHK_SLIDING_REG_COULOMB) ? L.C : (DIR == 0 ? L.Cx : L.Cy)[fi];
         o.taub = taub_face(P, L, Nf, lf, av, o.ub, Cf);
     }
     return o;
@@ -277,7 +284,8 @@ __device__ __forceinline__ FaceSums face_sums(const FaceOut &o) {
     return FaceSums{o.re, o.ub * o.taub, o.q * o.dh, o.q * o.dpw};
 }
 
-template <bool FROM_H, bool CHECK>
+// COEF: the law may have face coefficients (false: the launch knows that it has one for all faces).
+template <bool FROM_H, bool CHECK, bool COEF>
 __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P, const Sliding &L,
                                           const shk_state &s, const uint8_t *__restrict__ m8,
                                           const double *__restrict__ h_prev, double *partials, unsigned int *counter,
@@ -285,6 +293,7 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
     const int lane = threadIdx.x & 31, warps = B.n * (kTailThreads / 32);
     const int nsx = (nx + kTailCols - 1) / kTailCols, per = max(1, warps / nsx), th = (ny + per - 1) / per,
               strips = nsx * ((ny + th - 1) / th);
+    const double *const cx = COEF ? face_coef<0>(L, s) : nullptr, *const cy = COEF ? face_coef<1>(L, s) : nullptr;
     double red[2] = {0.0, 0.0};
     for (int st = B.id * (kTailThreads / 32) + (threadIdx.x >> 5); st < strips; st += warps) {
         const int ix = (st % nsx) * kTailCols - 1 + lane, y0 = (st / nsx) * th, y1 = min(y0 + th, ny);
@@ -316,11 +325,12 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
         FaceSums S;
         {
             const CellQ q = make_cell<FROM_H>(P, below);
-            const FaceOut o = face<FROM_H, 1>(P, L, s, c, y0 > 0, q, cur, cur, fs);
+            const FaceOut o = face<FROM_H, 1>(P, L, s, c, y0 > 0, q, cur, cur, fs, cy ? cy[c] : L.C);
             if (own) put_y(c, y0 > 0, o);
             S = face_sums(o);
         }
         for (int iy = y0; iy < y1; iy++, c += nx, fx += nx + 1) {
+            const double Cn = cy ? cy[c + nx] : L.C, Cw = cx ? cx[fx] : L.C;
             const double G = s.G[c], bb = s.b[c], hp = CHECK ? h_prev[c] : 0.0;
             // the next row's inputs
             const bool more = iy + 1 < y1;
@@ -330,7 +340,7 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
             const CellQ nxt = make_cell<FROM_H>(P, next_r);
             // north face
             const bool nint = iy + 1 < ny;
-            const FaceOut on = face<FROM_H, 1>(P, L, s, c + nx, nint, cur, nxt, cur, north_r);
+            const FaceOut on = face<FROM_H, 1>(P, L, s, c + nx, nint, cur, nxt, cur, north_r, Cn);
             if (own && (more || !nint)) put_y(c + nx, nint, on);
             const FaceSums Nf = face_sums(on);
             // west face
@@ -340,7 +350,7 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
             w.N = __shfl_up_sync(0xffffffffu, cur.N, 1);
             w.lam = __shfl_up_sync(0xffffffffu, cur.lam, 1);
             w.aub = __shfl_up_sync(0xffffffffu, cur.aub, 1);
-            const FaceOut ow = face<FROM_H, 0>(P, L, s, fx, xint, w, cur, ix > 0 ? w : cur, west_r);
+            const FaceOut ow = face<FROM_H, 0>(P, L, s, fx, xint, w, cur, ix > 0 ? w : cur, west_r, Cw);
             if (xown) {
                 if (xint && FROM_H) {
                     s.dhdx[fx] = ow.dh;
@@ -399,13 +409,13 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
     }
 }
 
-template <bool FROM_H, bool CHECK>
+template <bool FROM_H, bool CHECK, bool COEF>
 __global__ void __launch_bounds__(kTailThreads, kTailBlocksPerSm) k_tail(int nx, int ny, Params P, Sliding L, shk_state s,
                                                       const uint8_t *__restrict__ m8,
                                                       const double *__restrict__ h_prev, double *partials,
                                                       unsigned int *counter, PicDev *pic, const CgDev *after) {
     // (not a return: the flag arrives while the first rows do)
-    tail_body<FROM_H, CHECK>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic, cg_ended(after));
+    tail_body<FROM_H, CHECK, COEF>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic, cg_ended(after));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -602,7 +612,12 @@ int tail_blocks(int nx, int ny, int num_sms) {
     const long long blocks = (strips + kTailThreads / 32 - 1) / (kTailThreads / 32);
     return (int)std::max(1LL, std::min(blocks, (long long)num_sms * kTailBlocksPerSm));
 }
-static int tail_grid(const Ctx *c) { return tail_blocks(c->nx, c->ny, c->num_sms); }
+template <bool FROM_H, bool CHECK>
+static void run_tail(Ctx *c, const double *h_prev, PicDev *pic, const CgDev *after) {
+    auto kernel = c->SL.kind == SHK_SLIDING_REG_COULOMB ? k_tail<FROM_H, CHECK, false> : k_tail<FROM_H, CHECK, true>;
+    kernel<<<tail_blocks(c->nx, c->ny, c->num_sms), kTailThreads, 0, c->stream>>>(
+        c->nx, c->ny, c->P, c->SL, c->st, c->mask8, h_prev, c->partials, c->counter, pic, after);
+}
 
 int launch_initial_conditions(Ctx *c) {
     const int nx = c->nx, ny = c->ny, n = nx * ny;
@@ -622,8 +637,7 @@ int launch_initial_conditions(Ctx *c) {
     k_init_faces<<<flat_grid(c, nf), kThreads, 0, c->stream>>>(nx, ny, c->P, c->st);
     c->launches++;
     if ((rc = check_launch(c, "k_init_faces"))) return rc;
-    k_tail<false, false><<<tail_grid(c), kTailThreads, 0, c->stream>>>(nx, ny, c->P, c->SL, c->st, c->mask8, nullptr,
-                                                                       c->partials, c->counter, nullptr, nullptr);
+    run_tail<false, false>(c, nullptr, nullptr, nullptr);
     c->launches++;
     return check_launch(c, "k_tail<init>");
 }
@@ -651,14 +665,8 @@ int launch_export_mfls(Ctx *c, double *aP, double *aE, double *aW, double *aN, d
 }
 
 int launch_tail(Ctx *c, bool picard_check, const CgDev *after) {
-    if (picard_check)
-        k_tail<true, true><<<tail_grid(c), kTailThreads, 0, c->stream>>>(c->nx, c->ny, c->P, c->SL, c->st, c->mask8,
-                                                                        c->h_prev, c->partials, c->counter,
-                                                                        &c->dev->pic, after);
-    else
-        k_tail<true, false><<<tail_grid(c), kTailThreads, 0, c->stream>>>(c->nx, c->ny, c->P, c->SL, c->st, c->mask8,
-                                                                         nullptr, c->partials, c->counter, nullptr,
-                                                                         after);
+    if (picard_check) run_tail<true, true>(c, c->h_prev, &c->dev->pic, after);
+    else run_tail<true, false>(c, nullptr, nullptr, after);
     c->launches++;
     return check_launch(c, "k_tail");
 }
@@ -712,7 +720,7 @@ __global__ void __launch_bounds__(kTailThreads, kTailBlocksPerSm) k_ens_tail(Ens
     __shared__ EnsInst I;
     const Blk B = ens_stage(I, E, b2i, EF_TAIL);
     if (!I.pic_active) return;
-    tail_body<true, true>(B, I.nx, I.ny, I.P, I.SL, I.st, I.mask8, I.h_prev, I.partials, I.counter, I.pic);
+    tail_body<true, true, true>(B, I.nx, I.ny, I.P, I.SL, I.st, I.mask8, I.h_prev, I.partials, I.counter, I.pic);
 }
 
 // step_b!: gap update of the cells, then the face averages (two launches: the faces read
