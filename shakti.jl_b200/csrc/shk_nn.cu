@@ -17,6 +17,7 @@
 //   weight grad  dW[tap, co, ci] = sum_p dY[p, co] X[p + off(tap), ci]                (split over
 //                pixel chunks, Float32 atomics)
 // with zero padding at each image's border.
+#include <algorithm>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -638,8 +639,13 @@ __global__ void __launch_bounds__(kHxThreads, 1) k_conv3x3_hx(const __grid_const
 // channels at 32768 pixels).  Rows are padded to 80 bytes: ldmatrix's 8 rows fall on different banks.
 // 8 to 14 us per layer (cold); a form with 1024-pixel chunks and fragments built from 16-bit global loads
 // took 70 to 120.
-// grid = (pixel chunks, ceil(Cout/32) * ceil(Cin/32), 9).  VEC: 16-byte aligned tensors (else 16-bit
-// loads).
+// grid = (pixel ranges, ceil(Cout/32) * ceil(Cin/32), 9).  VEC: 16-byte aligned tensors (else loads of words
+// and halves).  RANGE: `chunks` chunks per block, one after another into the same sums, or an image smaller than
+// a chunk.  Large images need it: a block's end is 1024 atomics on a gradient of a few thousand elements, and at
+// 1024 x 1024 pixels of 16 channels one chunk per block took 696 us, four take 265 (512 us with the 16-bit
+// loads); 512 x 512 of 32 channels 176 and 86.  From 256 chunks of an image on: at 90 and 128 (24 x 24 x 40, 64
+// channels; 64 x 64 x 8, 128 channels) one chunk per block is the faster one, 37 against 41 us and 162 against
+// 169.  Four at most: 1024 pixels in one Float32 sum, as in the form before.
 // ---------------------------------------------------------------------------------------------
 constexpr int kWgPx = 256, kWgTile = 32, kWgPitch = 40;
 
@@ -649,56 +655,77 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const bf16 *
                  : "r"(su32(p)));
 }
 
-template <bool VEC>
+template <bool VEC, bool RANGE>
 __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ dY,
                                                        float *__restrict__ dW, int N, int H, int W, int Cin,
-                                                       int Cout) {
+                                                       int Cout, int chunks) {
     __shared__ __align__(16) bf16 sY[kWgPx * kWgPitch], sX[kWgPx * kWgPitch];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tap = blockIdx.z, dy = tap / 3 - 1, dx = tap % 3 - 1;
     const int tiles_ci = (Cin + kWgTile - 1) / kWgTile;
     const int co0 = (blockIdx.y / tiles_ci) * kWgTile, ci0 = (blockIdx.y % tiles_ci) * kWgTile;
-    const long long hw = (long long)H * W, P = N * hw, p0 = (long long)blockIdx.x * kWgPx;
-    // the chunk's first pixel; later ones are counted on from it
-    const long long n0 = p0 / hw;
-    const int q0 = (int)(p0 % hw), y0 = q0 / W, x0 = q0 % W;
+    const long long hw = (long long)H * W, P = N * hw;
     auto copy = [&](bf16 *dst, const bf16 *src, bool in) {
         if (VEC) {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(su32(dst)), "l"(src), "r"(in ? 16 : 0)
                          : "memory");
-        } else {
+        } else {  // eight elements from any even address: words where they are aligned, halves at the ends
+            uint32_t w[4] = {0, 0, 0, 0};
+            if (in && ((uintptr_t)src & 2) == 0) {
+                const uint32_t *q = reinterpret_cast<const uint32_t *>(src);
 #pragma unroll
-            for (int k = 0; k < 8; k++) dst[k] = in ? src[k] : __ushort_as_bfloat16(0);
+                for (int k = 0; k < 4; k++) w[k] = q[k];
+            } else if (in) {
+                const uint32_t *q = reinterpret_cast<const uint32_t *>(src + 1);
+                const uint32_t first = *reinterpret_cast<const uint16_t *>(src), a = q[0], b = q[1], c = q[2],
+                               last = *reinterpret_cast<const uint16_t *>(src + 7);
+                w[0] = first | a << 16;
+                w[1] = a >> 16 | b << 16;
+                w[2] = b >> 16 | c << 16;
+                w[3] = c >> 16 | last << 16;
+            }
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     };
-    for (int i = tid; i < kWgPx * (kWgTile / 8); i += 128) {
-        const int px = i / (kWgTile / 8), c = (i % (kWgTile / 8)) * 8;
-        const long long p = p0 + px;
-        const int xs = x0 + px, ys = y0 + xs / W, sx = xs % W + dx, sy = ys % H + dy;
-        const bool iny = p < P && co0 + c < Cout;
-        copy(sY + px * kWgPitch + c, iny ? dY + p * Cout + co0 + c : dY, iny);
-        const bool inx = p < P && ci0 + c < Cin && sx >= 0 && sx < W && sy >= 0 && sy < H;
-        const long long q = ((n0 + ys / H) * H + sy) * W + sx;
-        copy(sX + px * kWgPitch + c, inx ? X + q * Cin + ci0 + c : X, inx);
-    }
-    if (VEC) asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
     const int m0 = (warp & 1) * 16, c0 = (warp >> 1) * 16;  // this warp's 16 x 16 of the tile
-    if (co0 + m0 >= Cout || ci0 + c0 >= Cin) return;
+    const bool mine = co0 + m0 < Cout && ci0 + c0 < Cin;
     const int r = lane & 7, mat = lane >> 3;
     // matrices 0..3 of A: (k, m) = (0, 0), (0, 8), (8, 0), (8, 8); of B: (k, n) = (0, 0), (8, 0), (0, 8), (8, 8)
     const bf16 *pa = sY + ((mat >> 1) * 8 + r) * kWgPitch + m0 + (mat & 1) * 8;
     const bf16 *pb = sX + ((mat & 1) * 8 + r) * kWgPitch + c0 + (mat >> 1) * 8;
     float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    for (int ch = 0; ch < (RANGE ? chunks : 1); ch++) {
+        const long long p0 = ((long long)blockIdx.x * (RANGE ? chunks : 1) + ch) * kWgPx;
+        if (RANGE && p0 >= P) break;
+        // the chunk's first pixel; later ones are counted on from it
+        const long long n0 = p0 / hw;
+        const int q0 = (int)(p0 % hw), y0 = q0 / W, x0 = q0 % W;
+        const int px_end = RANGE ? (int)min((long long)kWgPx, (P - p0 + 15) / 16 * 16) : kWgPx;
+        if (RANGE && ch) __syncthreads();  // the previous chunk is read
+        for (int i = tid; i < px_end * (kWgTile / 8); i += 128) {
+            const int px = i / (kWgTile / 8), c = (i % (kWgTile / 8)) * 8;
+            const long long p = p0 + px;
+            const int xs = x0 + px, ys = y0 + xs / W, sx = xs % W + dx, sy = ys % H + dy;
+            const bool iny = p < P && co0 + c < Cout;
+            copy(sY + px * kWgPitch + c, iny ? dY + p * Cout + co0 + c : dY, iny);
+            const bool inx = p < P && ci0 + c < Cin && sx >= 0 && sx < W && sy >= 0 && sy < H;
+            const long long q = ((n0 + ys / H) * H + sy) * W + sx;
+            copy(sX + px * kWgPitch + c, inx ? X + q * Cin + ci0 + c : X, inx);
+        }
+        if (VEC) asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (!mine) continue;
 #pragma unroll 4
-    for (int k = 0; k < kWgPx; k += 16) {
-        uint32_t a[4], b[4];
-        ldmatrix_x4_trans(a, pa + k * kWgPitch);
-        ldmatrix_x4_trans(b, pb + k * kWgPitch);
-        const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
-        mma_bf16(acc[0], a, b0);
-        mma_bf16(acc[1], a, b1);
+        for (int k = 0; k < px_end; k += 16) {
+            uint32_t a[4], b[4];
+            ldmatrix_x4_trans(a, pa + k * kWgPitch);
+            ldmatrix_x4_trans(b, pb + k * kWgPitch);
+            const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+            mma_bf16(acc[0], a, b0);
+            mma_bf16(acc[1], a, b1);
+        }
     }
+    if (!mine) return;
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -1168,14 +1195,15 @@ SHK_API int shk_nn_conv3x3_wgrad(const void *X, const void *dY, float *dW, int N
                                  void *stream) {
     if (!X || !dY || !dW || Cin % 8 || Cout % 16) return SHK_BAD_ARG;
     const long long P = (long long)N * H * W;
-    dim3 grid((unsigned)((P + kWgPx - 1) / kWgPx),
-              (unsigned)(((Cout + kWgTile - 1) / kWgTile) * ((Cin + kWgTile - 1) / kWgTile)), 9);
-    if ((((uintptr_t)X | (uintptr_t)dY) & 15) == 0)
-        k_conv3x3_wgrad<true><<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W,
-                                                                      Cin, Cout);
-    else
-        k_conv3x3_wgrad<false><<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W,
-                                                                       Cin, Cout);
+    const unsigned tiles = (unsigned)(((Cout + kWgTile - 1) / kWgTile) * ((Cin + kWgTile - 1) / kWgTile));
+    const bool vec = (((uintptr_t)X | (uintptr_t)dY) & 15) == 0;
+    const long long px = (P + kWgPx - 1) / kWgPx;
+    const int chunks = (int)std::min(4LL, std::max(1LL, px / (vec ? 128 : 512)));
+    dim3 grid((unsigned)((px + chunks - 1) / chunks), tiles, 9);
+    const bool range = chunks > 1 || P <= kWgPx / 2;
+    auto kernel = vec ? (range ? k_conv3x3_wgrad<true, true> : k_conv3x3_wgrad<true, false>)
+                      : (range ? k_conv3x3_wgrad<false, true> : k_conv3x3_wgrad<false, false>);
+    kernel<<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16 *)X, (const bf16 *)dY, dW, N, H, W, Cin, Cout, chunks);
     return cudaGetLastError() == cudaSuccess ? SHK_OK : SHK_CUDA_ERROR;
 }
 
