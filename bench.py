@@ -39,8 +39,9 @@ UNIT = "timesteps/s"
 # Algorithmic bytes per cell of one CG iteration.  Jacobi (Float64): k_cg_A reads aP, aE, aN, r,
 # p_old and writes p_new, Ap; k_cg_B reads aP, p_new, Ap, x, r and writes x, r (14 words).  With the
 # multigrid preconditioner, k_cg_A reads z instead of r (7 words) and the x/r update is counted
-# with the V-cycle's first kernel (mg_vcycle_bytes).  The counts are the algorithm's: the kernels keep
-# the multigrid form's z as a Float32 value and move 4 bytes less on each side of it.
+# with the V-cycle's first kernel (mg_vcycle_bytes).  These count every Krylov vector as Float64; with
+# moved=True the functions below count what the default multigrid kernels move, whose z is stored as the
+# Float32 value it is (4 bytes less where it is written and where it is read).
 CG_BYTES = {"plain": 14 * 8, "fp32cg": 14 * 4, "multigrid": 7 * 8}
 FORMS = {"multigrid": "Float64 CG + Float32 aggregation-multigrid V-cycle preconditioner",
          "plain": "Float64 CG, Jacobi (the reference algorithm)",
@@ -234,31 +235,61 @@ def run_steps(shk, sim, n, record=None):
             record.append(dict(picard=ps.last_iter, converged=ps.converged, cg=ps.cg_iters_total))
 
 
-def mg_vcycle_bytes(nx, ny, fused=True):
+def mg_dims(nx, ny):
+    dims = [(nx, ny)]
+    while dims[-1] != (1, 1):
+        a, b = dims[-1]
+        dims.append(((a + 1) // 2, (b + 1) // 2))
+    return dims
+
+
+def bottom_level(dims):
+    """The finest level that k_mg_bottom takes (bottom_level and bot_fits in the library): levels of at most 64
+    cells in one warp, then up to three with columns of 1 and 2 cells and blocks of 8 per thread, as their
+    cells and bordered arrays fit."""
+    def fits(d, strip):
+        x, y = d
+        if strip == 0:
+            return x * y <= 64 and (x + 2) * (y + 2) <= 200
+        if strip == 1:
+            return x * y <= 512 and (x + 2) * (y + 2) <= 1600
+        if strip == 2:
+            return x * ((y + 1) // 2) <= 512 and (x + 2) * ((y + 1) // 2 * 2 + 2) <= 2100
+        return (x + 1) // 2 * ((y + 3) // 4) <= 512 and ((x + 1) // 2 * 2 + 4) * ((y + 3) // 4 * 4 + 2) <= 6200
+    lb, strips = len(dims) - 1, 0
+    while lb > 1 and fits(dims[lb - 1], 0) and len(dims) - lb < 8:
+        lb -= 1
+    while strips < 3 and lb > 1 and fits(dims[lb - 1], strips + 1):
+        lb, strips = lb - 1, strips + 1
+    return lb
+
+
+def mg_vcycle_bytes(nx, ny, fused=True, moved=False):
     """Algorithmic bytes of one V-cycle (all levels, nu = 2 sweeps per side).
     Fused level kernels (the default): level 0 (Float64 residual in, Float64 z out), per fine cell,
     descending half with the CG's r update folded in and its x update once per two iterations --
     62 B on average: r, Ap 16 B, activity flag 1, operator wD dP aE aN 16 in, new r 8, the level's
     iterate 4, coarse rhs 1 out, and every second iteration p, p_prev, x 24 B in and x 8 B out --
-    and ascending half 38 B (iterate 4, coarse iterate 1, flag 1, operator 16, r 8 in; z 8 out);
-    each coarse level above the bottom, per cell, 26 + 30 B (Float32 rhs).  Per-sweep kernels:
-    level 0 17 + 33 + 26 + 34 + 37 B, coarse levels 13 + 29 + 22 + 30 + 29 B.  The levels the
-    one-block bottom kernel takes (at most 1400 cells in all, 29 B per cell within 200 KiB) are
-    read once (operator 17 B + rhs 4 B per cell) and level lb's result written once (4 B)."""
-    dims = [(nx, ny)]
-    while dims[-1] != (1, 1):
-        a, b = dims[-1]
-        dims.append(((a + 1) // 2, (b + 1) // 2))
+    and ascending half 38 B (iterate 4, coarse iterate 1, flag 1, operator 16, r 8 in; z 8 out, 4 with
+    `moved`); each coarse level above the bottom, per cell, 26 + 30 B (Float32 rhs).  Per-sweep kernels:
+    level 0 17 + 33 + 26 + 34 + 37 B, coarse levels 13 + 29 + 22 + 30 + 29 B.  The levels of the
+    one-block bottom kernel are read once (operator 17 B + rhs 4 B per cell) and level lb's result written
+    once (4 B): with `moved` those that it takes, else those of at most 1400 cells in all, as the kernel
+    took when the count was set."""
+    dims = mg_dims(nx, ny)
     cells = [a * b for a, b in dims]
-    lb = len(dims) - 1
-    rest = 0
-    for l in range(len(dims) - 1, 0, -1):
-        rest += cells[l]
-        if rest * 29 > 200 * 1024 or rest > 1400:
-            break
-        lb = l
+    if moved:
+        lb = bottom_level(dims)
+    else:
+        lb = len(dims) - 1
+        rest = 0
+        for l in range(len(dims) - 1, 0, -1):
+            rest += cells[l]
+            if rest * 29 > 200 * 1024 or rest > 1400:
+                break
+            lb = l
     top, coarse = (100, 56) if fused else (147 + 48, 123)  # per-sweep: plus k_cg_B's 48 B
-    total = top * cells[0] if len(dims) > 1 else 37 * cells[0]
+    total = (top - 4 * (moved and fused)) * cells[0] if len(dims) > 1 else 37 * cells[0]
     for l in range(1, lb):
         total += coarse * cells[l]
     if len(dims) > 1:
@@ -266,11 +297,13 @@ def mg_vcycle_bytes(nx, ny, fused=True):
     return total
 
 
-def iteration_bytes(form, nx, ny):
+def iteration_bytes(form, nx, ny, moved=False):
     cells = nx * ny
     b = CG_BYTES[form] * cells
     if form == "multigrid":
-        b += mg_vcycle_bytes(nx, ny, fused=os.environ.get("SHK_MG_FUSED", "1") != "0")
+        kind = os.environ.get("SHK_MG_FUSED", "1")
+        moved = moved and kind == "1" and cells > 1  # (the other forms store z in Float64)
+        b += mg_vcycle_bytes(nx, ny, fused=kind != "0", moved=moved) - 4 * cells * moved
     return b
 
 
@@ -281,24 +314,24 @@ def iteration_bytes(form, nx, ny):
 PICARD_BYTES, GAP_BYTES = 43 * 8, 11 * 8
 
 
-def step_bytes(form, nx, ny, counts):
+def step_bytes(form, nx, ny, counts, moved=False):
     """Algorithmic bytes of the timed window per timestep: every Picard iteration's field work,
     every CG iteration of `form`, every gap step."""
     cells = nx * ny
-    total = (counts["picard_iters"] * PICARD_BYTES * cells + counts["cg_iters"] * iteration_bytes(form, nx, ny)
+    total = (counts["picard_iters"] * PICARD_BYTES * cells + counts["cg_iters"] * iteration_bytes(form, nx, ny, moved)
              + counts["steps"] * GAP_BYTES * cells)
     return total / max(counts["steps"], 1)
 
 
-def step_roofline(form, w, counts, ms_per_step, peaks):
-    b = step_bytes(form, w.nx, w.ny, counts)
+def step_roofline(form, w, counts, ms_per_step, peaks, moved=False):
+    b = step_bytes(form, w.nx, w.ny, counts, moved)
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = b / (ms_per_step / 1e3) / 1e9
     return {"bound": "hbm", "bytes_per_step": int(b), "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4),
             "accounting": (f"per timestep: {counts['picard_iters']}/{counts['steps']} Picard iterations x "
                            f"{PICARD_BYTES} B/cell (assembly, tail, check) + {counts['cg_iters']}/{counts['steps']} "
-                           f"CG iterations x {iteration_bytes(form, w.nx, w.ny) / (w.nx * w.ny):.1f} B/cell + "
+                           f"CG iterations x {iteration_bytes(form, w.nx, w.ny, moved) / (w.nx * w.ny):.1f} B/cell + "
                            f"{GAP_BYTES} B/cell (gap step)"),
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6650 GB/s (of fallback)"}
 
@@ -340,7 +373,7 @@ def measure_cg_iteration(shk, sim, form, short=20, long=220):
 
 def roofline_for(shk, sim, form, w, peaks):
     it_ms, it_n = measure_cg_iteration(shk, sim, form)
-    nbytes = iteration_bytes(form, w.nx, w.ny)
+    nbytes = iteration_bytes(form, w.nx, w.ny, moved=True)
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = nbytes / (it_ms / 1e3) / 1e9
     kernel = {"plain": "k_cg_matvec_t<true> + k_cg_B (one Jacobi-PCG iteration, Float64: the p update with "
@@ -530,7 +563,8 @@ def ours(args, world, rank, local, pg):
         "config": bench_config(w, args, world),
         "form": FORMS[args.form],
         "roofline": roofline,
-        "step_roofline": step_roofline(args.form, w, counts_of(main["rec"]), main["ms_max"] / args.steps, peaks),
+        "step_roofline": step_roofline(args.form, w, counts_of(main["rec"]), main["ms_max"] / args.steps, peaks,
+                                       moved=True),
         "plain_fp64_gpu": plain,
         "cpu_baseline": cpu,
         "e2e": e2e,
