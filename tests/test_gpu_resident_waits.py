@@ -1,4 +1,6 @@
 """The bounded waits of the resident solves (shk_resident.cuh), cut short."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -157,6 +159,10 @@ def test_a_part_of_the_device(shk, cuda, monkeypatch, nx, ny, precond):
     kw = dict(rtol=0.0, itmax=20)
     want, ref = Problem(shk, monkeypatch, nx, ny, precond, resident=False).solve(**kw)
     part = cuda.cuda.GreenContext.create(16, 0)
-    with cuda.cuda.stream(part.Stream()):
+    stream = part.Stream()
+    with cuda.cuda.stream(stream):
         h, st = Problem(shk, monkeypatch, nx, ny, precond).solve(**kw)
+    gc.collect()  # the solver contexts synchronise their stream when they go: before it does
+    cuda.cuda.synchronize()
+    del stream, part
     assert (st.niter, st.status) == (ref.niter, ref.status) and np.array_equal(h, want)
