@@ -289,7 +289,7 @@ template <bool FROM_H, bool CHECK, bool COEF>
 __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P, const Sliding &L,
                                           const shk_state &s, const uint8_t *__restrict__ m8,
                                           const double *__restrict__ h_prev, double *partials, unsigned int *counter,
-                                          PicDev *pic, bool keep = true) {
+                                          PicDev *pic) {
     const int lane = threadIdx.x & 31, warps = B.n * (kTailThreads / 32);
     const int nsx = (nx + kTailCols - 1) / kTailCols, per = max(1, warps / nsx), th = (ny + per - 1) / per,
               strips = nsx * ((ny + th - 1) / th);
@@ -297,8 +297,8 @@ __device__ __forceinline__ void tail_body(Blk B, int nx, int ny, const Params &P
     double red[2] = {0.0, 0.0};
     for (int st = B.id * (kTailThreads / 32) + (threadIdx.x >> 5); st < strips; st += warps) {
         const int ix = (st % nsx) * kTailCols - 1 + lane, y0 = (st / nsx) * th, y1 = min(y0 + th, ny);
-        const bool own = keep && lane >= 1 && lane <= kTailCols && ix < nx;
-        const bool xown = own || (keep && lane >= 1 && ix == nx);   // writes its west face (ix = nx: the domain's east edge)
+        const bool own = lane >= 1 && lane <= kTailCols && ix < nx;
+        const bool xown = own || (lane >= 1 && ix == nx);   // writes its west face (ix = nx: the domain's east edge)
         const bool xint = ix > 0 && ix < nx;
         // Lanes beyond the grid read the nearest cell and face, rows beyond it the last row: every load
         // is in bounds without a test, and what those lanes compute is not written.
@@ -414,8 +414,8 @@ __global__ void __launch_bounds__(kTailThreads, kTailBlocksPerSm) k_tail(int nx,
                                                       const uint8_t *__restrict__ m8,
                                                       const double *__restrict__ h_prev, double *partials,
                                                       unsigned int *counter, PicDev *pic, const CgDev *after) {
-    // (not a return: the flag arrives while the first rows do)
-    tail_body<FROM_H, CHECK, COEF>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic, cg_ended(after));
+    if (!cg_ended(after)) return;
+    tail_body<FROM_H, CHECK, COEF>(grid_blk(), nx, ny, P, L, s, m8, h_prev, partials, counter, pic);
 }
 
 // ---------------------------------------------------------------------------------------------
