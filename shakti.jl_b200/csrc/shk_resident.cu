@@ -5,9 +5,12 @@
 // which is less than the 148 SMs hold in registers and shared memory (71 MB).  Launched as two (Jacobi)
 // or six (Chebyshev) kernels per iteration, such a solve spends its time on launches, on block
 // start-up and on moving those arrays through L2: 20 us per iteration at 201 x 150 and 31 us at 1024^2
-// with Jacobi, 25 and 84 us at 64^2 and 1024^2 with Chebyshev(4); here it is 4.4 and 11.8, 6.8 and 26.  Here one block per SM (a cooperative
-// launch) owns a strip of whole rows for the entire solve; each thread owns two adjacent columns of R
-// rows, with r, p and A p in registers, the operator (and x for the largest R) in shared memory, and
+// with Jacobi, 25 and 84 us at 64^2 and 1024^2 with Chebyshev(4); here it is 4.4 and 11.8, 6.8 and 26 (a step's
+// Picard work and Lanczos bounds not counted).  One block per SM (a cooperative launch) owns a strip of whole
+// rows for the entire solve; each thread owns two adjacent columns of R rows, with the operator in shared
+// memory and p, A p (z) in registers; r and x are there too for R <= 4 (Jacobi) and R <= 2 (Chebyshev).  For
+// larger R the vectors that do not fit lie in shared memory (r; ResSmem) or in a scratch array in L2 in the
+// threads' own order (x, and at R = 7 of Chebyshev r and p), each read and written once an iteration.  Otherwise
 // only sums and strip-edge rows cross L2.
 //
 // An iteration has the two all-block sums of CG (p'Ap, then r'z and r'r) and, per application of the
@@ -17,8 +20,8 @@
 // its reader, and a block learns every other block's partial one L2 hop after it was written.  A
 // buffer is rewritten only two events later, when its readers have provably read it (they contributed
 // to the event in between).  Each block adds the partials in the same order, so all blocks take the
-// same decisions and stop together.  Polls are bounded; a wait that runs out makes the solve report a
-// fault.
+// same decisions and stop together.  Polls are bounded, and they begin only when every block of the launch
+// runs; how a solve starts, and how it ends when a wait runs out, is told in shk_resident.cuh.
 //
 // Element for element the arithmetic is that of the general kernels in shk_krylov.cu (same formulas,
 // same order, unfused); only the order of the sums differs.
@@ -87,8 +90,7 @@ struct ResSmem {
     // rows with a stored reciprocal of aP, a fourth operator array: all that fit
     static constexpr int recip = R <= 4 ? R : (CHEB ? R - 1 : 0);
     static constexpr int op = 6 * R + 2 * recip;   // operator planes
-    static constexpr int vecs = (rmode == V_SMEM) + (xmode == V_SMEM);
-    static constexpr size_t planes = (size_t)(op + 2 * vecs * R) * kResThreads;
+    static constexpr size_t planes = (size_t)(op + 2 * (rmode == V_SMEM) * R) * kResThreads;
     static constexpr size_t edges = (size_t)bufs * 2 * R * kResWarps;
     static constexpr size_t rows = R > 4 ? 0 : (size_t)bufs * 4 * kResThreads;  // R = 7: one row group
     static constexpr size_t bytes = (planes + edges + rows) * sizeof(double);
@@ -120,7 +122,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     ResVec<L::xmode, R> x;
     ResVec<L::pmode, R> pm;  // V_REG: unused, p itself is in registers
     r.s = sm + L::op * T + S.tid;
-    x.s = sm + (L::op + 2 * R * (L::rmode == V_SMEM)) * T + S.tid;
     x.stride = pm.stride = r.stride = (size_t)gridDim.x * T;
     x.g = A.vec + (size_t)blockIdx.x * T + S.tid;
     pm.g = x.g + R * x.stride;

@@ -105,6 +105,8 @@ __device__ __forceinline__ void wait_limit(const ResComm &A, volatile ResWait &W
 }
 
 // ---- tagged words -------------------------------------------------------------------------------
+// Half a value and a flag in each 8 bytes, both pairs in one 16-byte access: the word format of NCCL's
+// low-latency (LL) protocol.
 __device__ __forceinline__ void ll_store(uint4 *p, double v, unsigned tag) {
     asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(__double2loint(v)), "r"(tag),
                  "r"(__double2hiint(v)), "r"(tag)
