@@ -186,12 +186,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
     volatile ResWait &W = sh.wait;
     if (tid == 0) {
         sh.cg = A.init;
-        wait_limit(A, W, 0);
-        sh.tag0 = res_arrive(A);
+        wait_start(A, sh.wait);
+        sh.kept = res_start(A, sh.tag0);
     }
     __syncthreads();
+    if (!sh.kept) return;
     const unsigned tag0 = sh.tag0;
-    if (tag0 == kResLost) return;  // lost before this block started
     unsigned st = tag0, vt = tag0, ht = tag0;  // tags of sums, V-cycles and row exchanges
     auto nothing = [&]() {};
     CgScalars &sc = sh.sc;
@@ -202,9 +202,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         BotShared &M = *reinterpret_cast<BotShared *>(smem);
         BotOp O;
         bot_load(A.bp, M, O);
-        if (tid == 0) sh.kept = res_started(A, tag0);
         __syncthreads();
-        if (!sh.kept) return;
         double v3[3] = {0.0, 0.0, 0.0}, v1[1] = {0.0}, v2[2] = {0.0, 0.0};
         for (bool first = true;; first = false) {  // (one place for the V-cycle: its registers stay registers)
             vt++;
@@ -233,12 +231,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
                 A, sh, lane, warp, v1, rb, ++st, nothing,
                 [&](double (&t)[1]) {
                     scalars_alpha(sc, t[0], A.eps_curv);
-                    wait_limit(A, W, sc.iter + 1);
+                    wait_iteration(sh.wait, (int)sc.iter + 1);
                 },
                 [](double (&)[1]) {});
             if (!ok || sc.done) break;
         }
-        if (!ok && tid == 0) res_end(A, tag0, kResLost, false, []() {});
+        if (!ok && tid == 0) res_end(A, tag0, kResLost, false);
         return;
     }
 
@@ -309,10 +307,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
         for (int x = tid; x < M.nx; x += T) M.N[x] = M.y0 > 0 ? V.aN[(size_t)(M.y0 - 1) * M.nx + x] : 0.0f;
         for (int i = tid; i < 2 * (M.n + 2 * M.nx); i += T) M.X0[i] = 0.0f;
     }
-
-    if (tid == 0) sh.kept = res_started(A, tag0);
-    __syncthreads();
-    if (!sh.kept) return;
 
     double r[R][2], p[R][2], q[R][2], xr[XG ? 1 : R][2];
     double rs[2] = {0.0, 0.0}, rn[2] = {0.0, 0.0};  // r on the rows below and above the strip
@@ -650,7 +644,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
             A, sh, lane, warp, v, rb, ++st, [&]() { recv64(as, an); },
             [&](double (&t)[1]) {
                 scalars_alpha(sc, t[0], A.eps_curv);
-                wait_limit(A, W, sc.iter + 1);
+                wait_iteration(sh.wait, (int)sc.iter + 1);
             },
             [](double (&)[1]) {});
         if (!ok || sc.done) break;
@@ -665,16 +659,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_mg_resident(const __grid_con
     }
 
     // ---- h = x + x0 (the row exchanges are the most frequent events: their tag is the last) ----------------
-    if (tid == 0) sh.kept = res_end(A, tag0, ht, ok, [&]() { *A.cg = scalars_record(sc, sh.cg); });
+    if (tid == 0) sh.kept = res_end(A, tag0, ht, ok);
     __syncthreads();
-    if (!sh.kept) return;
-#pragma unroll
-    for (int j = 0; j < R; j++) {
-        if (!valid(j, 0)) continue;
-        const double2 xj = XG ? xg[(size_t)j * G * T] : make_double2(xr[XG ? 0 : j][0], xr[XG ? 0 : j][1]);
-        A.h[cell(j, 0)] = xj.x + A.x0[cell(j, 0)];
-        if (valid(j, 1)) A.h[cell(j, 1)] = xj.y + A.x0[cell(j, 1)];
-    }
+    if (sh.kept == kResDropped) return;
+    add_to_head<R>(A, nx, ny, A.x0, A.h, [&](int j) {
+        return XG ? xg[(size_t)j * G * T] : make_double2(xr[XG ? 0 : j][0], xr[XG ? 0 : j][1]);
+    });
+    if (tid == 0 && sh.kept == kResSettled) *A.cg = scalars_record(sc, sh.cg);
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -130,16 +130,16 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     int hb = 0, rb = 0, sb = 0;  // halo, sum and shared-memory buffers in turn
     if (S.tid == 0) {
         sh.cg = A.init;
-        wait_limit(A, sh.wait, 0);
-        sh.tag0 = res_arrive(A);
+        wait_start(A, sh.wait);
+        sh.kept = res_start(A, sh.tag0);
         if (CHEB) {
             ch.lam_min = A.cheb->lam_min;
             ch.lam_max = A.cheb->lam_max;
         }
     }
     __syncthreads();
+    if (!sh.kept) return;
     unsigned tag = sh.tag0;
-    if (tag == kResLost) return;  // lost before this block started
     auto valid = [&](int j, int e) { return S.act && S.c0 + e < nx && S.row0 + j < ny; };
     auto cell = [&](int j, int e) { return (size_t)(S.row0 + j) * nx + S.c0 + e; };
     // a / aP; r / aP keeps an infinite r (after an operator application an infinite value ends in NaN anyway)
@@ -177,9 +177,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
         }
     S.aS0 = S.row0 > 0 && valid(0, 0) ? A.aN[cell(-1, 0)] : 0.0;
     S.aS1 = S.row0 > 0 && valid(0, 1) ? A.aN[cell(-1, 1)] : 0.0;
-    if (S.tid == 0) sh.kept = res_started(A, sh.tag0);
-    __syncthreads();
-    if (!sh.kept) return;
     // v on the thread's rows -> the operator's inputs around it (block barrier inside)
     auto share = [&](const double (&v)[R][2], double (&s)[2], double (&n)[2]) {
         if (CHEB) sb ^= 1;
@@ -409,7 +406,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
             A, sh, S.lane, S.warp, v, rb, ++tag, nothing,
             [&](double (&t)[1]) {
                 scalars_alpha(sc, t[0], A.eps_curv);
-                wait_limit(A, sh.wait, sc.iter + 1);
+                wait_iteration(sh.wait, (int)sc.iter + 1);
             },
             [](double (&)[1]) {});
         if (!ok || sc.done) break;
@@ -433,26 +430,20 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     }
 
     // ---- h = x + x0 ----------------------------------------------------------------------------------
-    if (S.tid == 0)
-        sh.kept = res_end(A, sh.tag0, tag, ok, [&]() {
-            *A.cg = scalars_record(sc, sh.cg);
-            if (CHEB) {
-                A.cheb->est_min = ch.est_min;
-                A.cheb->est_max = ch.est_max;
-                A.cheb->adopted = ch.adopted;
-                A.cheb->lam_min = ch.lam_min;
-                A.cheb->lam_max = ch.lam_max;
-                cheb_coefficients(ch.lam_min, ch.lam_max, kMaxChebDegree, A.cheb->calpha, A.cheb->cbeta);
-            }
-        });
+    if (S.tid == 0) sh.kept = res_end(A, sh.tag0, tag, ok);
     __syncthreads();
-    if (!sh.kept) return;
-#pragma unroll
-    for (int j = 0; j < R; j++) {
-        if (!valid(j, 0)) continue;
-        const double2 xj = x.get(j);
-        A.h[cell(j, 0)] = xj.x + A.x0[cell(j, 0)];
-        if (valid(j, 1)) A.h[cell(j, 1)] = xj.y + A.x0[cell(j, 1)];
+    if (sh.kept == kResDropped) return;
+    add_to_head<R>(A, nx, ny, A.x0, A.h, [&](int j) { return x.get(j); });
+    if (S.tid == 0 && sh.kept == kResSettled) {
+        *A.cg = scalars_record(sc, sh.cg);
+        if (CHEB) {
+            A.cheb->est_min = ch.est_min;
+            A.cheb->est_max = ch.est_max;
+            A.cheb->adopted = ch.adopted;
+            A.cheb->lam_min = ch.lam_min;
+            A.cheb->lam_max = ch.lam_max;
+            cheb_coefficients(ch.lam_min, ch.lam_max, kMaxChebDegree, A.cheb->calpha, A.cheb->cbeta);
+        }
     }
 }
 

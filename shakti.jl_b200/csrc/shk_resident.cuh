@@ -19,7 +19,7 @@ struct ResComm {
     uint4 *red;              // [2][groups][4] tagged partials
     uint4 *halo;             // [2][groups][2][2 * txp] tagged strip-edge rows
     CgDev *cg;
-    unsigned int *epoch;     // tags used so far: the solve's word (res_arrive)
+    unsigned int *epoch;     // tags used so far: the solve's word (res_start)
     unsigned int *arrived;   // blocks that have started
     int spin;                // polls before a wait gives up
     int start_spin;          // polls before a block stops waiting for the launch's other blocks to start
@@ -40,19 +40,17 @@ constexpr unsigned kResRunning = 1u << 31, kResLost = ~0u;
 // kernel may hold some of their SMs for as long as it likes.  So no block polls for another's words before all
 // of them have started, and when that takes too long (start_spin) the solve is lost before it began and the
 // host turns to the general kernels, whose blocks wait for nobody.  The last block to arrive starts the
-// solve; the blocks load their operator meanwhile.  One thread of each block calls these.
-__device__ __forceinline__ unsigned res_arrive(const ResComm &A) {  // returns t, or kResLost
+// solve.  One thread of each block; false: the block leaves.
+__device__ __forceinline__ bool res_start(const ResComm &A, unsigned &tag0) {
     const unsigned t = *(volatile unsigned *)A.epoch;
-    if (t == kResLost || A.test_absent == (int)blockIdx.x) return kResLost;
+    tag0 = t;
+    if (t == kResLost || A.test_absent == (int)blockIdx.x) return false;
     __threadfence();
     if (atomicAdd(A.arrived, 1u) + 1 == gridDim.x) {
         *(volatile unsigned *)A.arrived = 0;
         __threadfence();
         atomicCAS(A.epoch, t, t | kResRunning);
     }
-    return t;
-}
-__device__ __forceinline__ bool res_started(const ResComm &A, unsigned t) {
     for (int i = 0;; i++) {
         const unsigned w = *(volatile unsigned *)A.epoch;
         if (w != t) return w == (t | kResRunning);
@@ -68,40 +66,41 @@ __device__ __forceinline__ bool res_started(const ResComm &A, unsigned t) {
 
 // Ending.  The outcome is settled by the first block that swaps the word: to the tags that it used when it has
 // completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here and
-// writes its rows of the head only if the solve was not lost; a block whose wait for the last sum ran out
+// writes its rows of the head only if the solve was not lost (one thread of each block calls this); a block whose wait for the last sum ran out
 // when another has completed it writes them too, since it has contributed to that sum and its x is final.
 // (A sum that completes has every block's partial, so no later wait can be the one that ran out.)
-// `record` is run by the one that settles a completed solve.
-template <typename Record>
-__device__ __forceinline__ bool res_end(const ResComm &A, unsigned t, unsigned last, bool ok, Record record) {
+// The one that settles a completed solve (kResSettled) writes its record.
+enum { kResDropped = 0, kResKept, kResSettled };
+__device__ __forceinline__ int res_end(const ResComm &A, unsigned t, unsigned last, bool ok) {
     const unsigned to = ok ? last : kResLost, was = atomicCAS(A.epoch, t | kResRunning, to);
-    if (was != (t | kResRunning)) return was != kResLost;
-    if (ok) {
-        record();
-    } else {
-        A.cg->fault = kFaultWait;
-        A.cg->done = 1;
-    }
-    return ok;
+    if (was != (t | kResRunning)) return was != kResLost ? kResKept : kResDropped;
+    if (ok) return kResSettled;
+    A.cg->fault = kFaultWait;
+    A.cg->done = 1;
+    return kResDropped;
 }
 
 // A block's waits (in its shared memory): one that runs out makes the whole block leave.
 struct ResWait {
     int abort;               // a wait of this block ran out
     int spin;                // polls that a wait has
+    int test_at, test_spin;  // tests: before the last sum of this iteration, this many (0: never)
 };
 __device__ __forceinline__ bool wait_over(volatile ResWait &W, int polls) {
     if (polls < W.spin && !W.abort) return false;
     W.abort = 1;
     return true;
 }
-// One thread: the block's limit at the start (iter = 0), and before the last sum of iteration `iter`.
-__device__ __forceinline__ void wait_limit(const ResComm &A, volatile ResWait &W, long long iter) {
-    if (iter == 0) {
-        W.abort = 0;
-        W.spin = A.spin;
-    }
-    if (iter == A.test_iter && (A.test_block < 0 || A.test_block == (int)blockIdx.x)) W.spin = A.test_spin;
+// One thread, at the start and before an iteration's last sum.
+__device__ __forceinline__ void wait_start(const ResComm &A, ResWait &W) {
+    const bool test = A.test_block < 0 || A.test_block == (int)blockIdx.x;
+    W.abort = 0;
+    W.spin = test && A.test_iter == 0 ? A.test_spin : A.spin;
+    W.test_at = test && A.test_iter > 0 ? A.test_iter : 0;
+    W.test_spin = A.test_spin;
+}
+__device__ __forceinline__ void wait_iteration(ResWait &W, int iter) {
+    if (iter == W.test_at) W.spin = W.test_spin;
 }
 
 // ---- tagged words -------------------------------------------------------------------------------
@@ -138,7 +137,7 @@ struct ResSums {
     CgScalars sc;
     ResWait wait;
     unsigned tag0;               // tags used before this solve
-    int kept;                    // the solve has started; at the end: it was not lost
+    int kept;                    // the solve has started; at the end: its outcome (res_end)
     int left;                    // wait.abort as the last sum left it, the same for every thread
 };
 
@@ -310,12 +309,12 @@ __device__ __forceinline__ void recv_rows(const ResComm &A, const Strip<R> &S, i
     const long blk = blockIdx.x;
     const uint4 *ps = base + (blk - 1) * (long)per + 2 * A.txp, *pn = base + (blk + 1) * (long)per;
     bool s0 = !S.south, s1 = s0, n0 = !S.north, n1 = n0;
-    for (int i = 0;; i++) {
+    for (int i = 0; !(s0 && s1 && n0 && n1); i++) {
         if (!s0) s0 = ll_try(ps, tag, s[0]);
         if (!s1) s1 = ll_try(ps + 1, tag, s[1]);
         if (!n0) n0 = ll_try(pn, tag, n[0]);
         if (!n1) n1 = ll_try(pn + 1, tag, n[1]);
-        if ((s0 && s1 && n0 && n1) || wait_over(W, i)) break;
+        if (!(s0 && s1 && n0 && n1) && wait_over(W, i)) break;
     }
 }
 
@@ -347,10 +346,11 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
     uint4 *slots = A.red + (size_t)buf * G * 4;
     double t[NV];
     if (warp < 2) {
+        const int lost = *(volatile int *)&sh.wait.abort;
 #pragma unroll
         for (int k = 0; k < NV; k++) t[k] = sum16(sh.wred[k], lane);
         // (a block whose wait ran out adds nothing: a sum that completes is one of whole partials)
-        if (warp == 0 && !alone && (int)blockIdx.x < G && !*(volatile int *)&sh.wait.abort) {
+        if (warp == 0 && !alone && (int)blockIdx.x < G && !lost) {
 #pragma unroll
             for (int k = 0; k < NV; k++)
                 if (lane == k) ll_store(slots + blockIdx.x * 4 + k, t[k], tag);
@@ -383,13 +383,31 @@ __device__ __forceinline__ bool all_sum(const ResComm &A, ResSums &sh, int lane,
             for (int k = 0; k < NV; k++) t[k] = sum16(sh.wsum[k], lane);
         }
     }
-    if (warp == 0 && lane == 0) {
-        sh.left = *(volatile int *)&sh.wait.abort;
-        fin(t);
-    }
+    if (warp == 0 && lane == 0) fin(t);
+    if (warp == 2 && lane == 0) sh.left = *(volatile int *)&sh.wait.abort;
     if (warp == 1 && lane == 0) fin2(t);
     __syncthreads();
     return !*(volatile int *)&sh.left;
+}
+
+// h = x + x0 on the thread's cells, x(j) its columns of row j.  The cells' coordinates are formed anew from a
+// thread index that the compiler takes for another value: kept from the start, they and what depends on them
+// hold registers through the iterations (spill loads of the 7-row Jacobi solve 188 B a thread with
+// them, 72 without: 11.3 and 11.0 us an iteration at 1024 x 1024).
+template <int R, typename X>
+__device__ __forceinline__ void add_to_head(const ResComm &A, int nx, int ny, const double *x0, double *h, X x) {
+    int tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int c0 = 2 * (tid % A.txp), gy = tid / A.txp, row0 = ((int)blockIdx.x * A.ty + gy) * R;
+    if (gy >= A.ty || c0 >= nx) return;
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        if (row0 + j >= ny) continue;
+        const double2 v = x(j);
+        const size_t c = (size_t)(row0 + j) * nx + c0;
+        h[c] = v.x + x0[c];
+        if (c0 + 1 < nx) h[c + 1] = v.y + x0[c + 1];
+    }
 }
 
 } // namespace shk
