@@ -92,6 +92,9 @@ struct DevScalars {
 // general kernels take its place.
 constexpr int kFaultWait = 1, kFaultNotStarted = 2;
 constexpr int kNotStarted = -1000;
+// Solves that the general kernels take after one that did not start: on a device whose SMs another stream holds,
+// the wait for them is paid once in so many.
+constexpr int kHoldSolves = 32;
 
 // Geometry of the resident solve (shk_resident.cu): rows per thread, threads per row group, row
 // groups per block, blocks (0: the grid does not fit).
@@ -186,6 +189,7 @@ struct Ctx {
     bool res_restart = false; // its tags start over at the next solve
     int res_spin = 1 << 21;   // polls before one of its waits gives up (about 1 s)
     int res_start_spin = 1 << 16;           // and before it gives up on blocks that have not started (about 40 ms)
+    int res_hold = 0;                       // solves left to the general kernels after one that did not start
     int res_test_absent = -1;               // tests: ResComm's
     const double *res_ws = nullptr;         // the warm start of the last resident solve
     int res_test_spin = -1, res_test_block = -1, res_test_iter = 0; // tests: ResComm's (-1: none)

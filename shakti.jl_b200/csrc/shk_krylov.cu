@@ -1098,6 +1098,7 @@ int collect_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st) {
         c->res_restart = true;
         if (g.fault == kFaultNotStarted) {
             c->ws_x0 = c->res_ws;
+            c->res_hold = kHoldSolves;
             return kNotStarted;
         }
         return fail(c, SHK_CUDA_ERROR, res_serves(c, o) || mg_res_serves(c, o)
@@ -1147,6 +1148,10 @@ int run_cg(Ctx *c, const shk_cg_opts *o, shk_cg_stats *st, bool *deferred, bool 
             return fail(c, SHK_BAD_ARG, "chebyshev nsteps must be in [2, 64]");
     }
     // the whole solve in one persistent kernel where the grid's Krylov state fits on the chip
+    if (resident && c->res_hold > 0 && (res_serves(c, o) || mg_res_serves(c, o))) {
+        c->res_hold--;
+        resident = false;
+    }
     if (resident && (res_serves(c, o) || mg_res_serves(c, o))) {
         const CgDev init = make_cg_init(o, n, false, 0.0);
         const double *x0 = ws ? ws : c->st.h;

@@ -128,6 +128,22 @@ def test_a_solve_that_cannot_start_runs_by_the_general_kernels(shk, cuda, monkey
         assert cuda.equal(b[5][f], t), f
 
 
+@pytest.mark.parametrize("nx,ny,precond", [(201, 150, "jacobi"), (64, 64, "chebyshev"), (200, 150, "multigrid")])
+def test_the_wait_for_a_start_is_paid_once_in_a_while(shk, cuda, monkeypatch, nx, ny, precond):
+    """After a solve that could not start, the context's next 32 do not try (each try waits about 40 ms); the one
+    after them does: it launches one kernel more."""
+    q = Problem(shk, monkeypatch, nx, ny, precond, ABSENT=0)
+    ls, counts = q.solver(rtol=0.0, itmax=3), []
+    for _ in range(36):
+        n = ls.ctx.launches()
+        q.s.h.copy_(q.h0)
+        shk.solve_elliptic_linear_system(ls, q.s, q.g, q.p, shk.Arithmetic(), q.sl)
+        counts.append(ls.ctx.launches() - n)
+    general = counts[1]
+    assert [k for k, c in enumerate(counts) if c > general] == [0, 33]
+    assert all(c == general for k, c in enumerate(counts) if k not in (0, 33))
+
+
 def test_two_solves_at_once(shk, cuda, monkeypatch):
     """Two host threads on two streams: each gets its own solution, whether the two launches follow one
     another or one gives way to the general kernels (to 1e-9, as between the two forms)."""
