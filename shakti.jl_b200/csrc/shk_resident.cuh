@@ -65,9 +65,9 @@ __device__ __forceinline__ bool res_start(const ResComm &A, unsigned &tag0) {
 }
 
 // Ending.  The outcome is settled by the first block that swaps the word: to the tags that it used when it has
-// completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here and
-// writes its rows of the head only if the solve was not lost (one thread of each block calls this); a block whose wait for the last sum ran out
-// when another has completed it writes them too, since it has contributed to that sum and its x is final.
+// completed the last sum, or to kResLost when a wait of its own ran out.  Every block ends here (one thread of it)
+// and writes its rows of the head only if the solve was not lost; a block whose wait for the last sum ran out when
+// another has completed it writes them too, since it has contributed to that sum and its x is final.
 // (A sum that completes has every block's partial, so no later wait can be the one that ran out.)
 // The one that settles a completed solve (kResSettled) writes its record.
 enum { kResDropped = 0, kResKept, kResSettled };
